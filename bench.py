@@ -1163,7 +1163,7 @@ def kernel_case(name):
             else:
                 ck.knn_learned(rec, q, 16, m, "stack_based", layout=lay, world_bounds=wb,
                                scale=1.2)
-    elif name == "heap":  # k = 64: knn_fast_heap_kernel
+    elif name == "heap":  # k = 64: knn_fast_kernel with a 65-slot list
         rec, wb, lay = _gmm_tree(ck)
         q = gmm_q(1_000_000)
         for _ in range(2):

@@ -418,11 +418,12 @@ static int query_impl(cukd_batch_plan_s *p, const float *pts, const float *bound
     fa.q = a;
     fa.kk = p->params.k;
     fa.fcp = false;
+    fa.method = p->params.method;
     CKB_CUDA(cudaMemsetAsync(p->ctr, 0, 2 * sizeof(int), st));
     fa.work = p->ctr;
     fa.fb_count = p->ctr + 1;
     fa.fb_list = p->fb_list;
-    CKB_TRY(run_fast(fa, D, st));
+    CKB_TRY(run_fast(fa, CUKD_FLOAT32, D, st));
     if (p->params.d_reordered_count)
       CKB_CUDA(cudaMemcpyAsync(p->params.d_reordered_count, fa.fb_count, sizeof(int),
                                cudaMemcpyDeviceToDevice, st));

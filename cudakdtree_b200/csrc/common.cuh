@@ -223,6 +223,15 @@ inline bool make_layout(const cukd_layout *l, Layout *out)
   return true;
 }
 
+// Whether a node can be read as one 16-byte load: 16-byte records whose
+// point comes first and whose dim, if explicit, is the last word, in an
+// array that starts on a 16-byte boundary.
+inline bool vec16_records(const void *tree, int stride, int poff, int doff, int D)
+{
+  return stride == 16 && poff == 0 && (doff < 0 || doff == 12) && D <= 3 &&
+         (reinterpret_cast<uintptr_t>(tree) & 15u) == 0;
+}
+
 inline int64_t div_up(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Largest tree the traversals accept: their node indices are 32-bit ints (as

@@ -1,6 +1,8 @@
 // Fast exact kNN / FCP path (fast.cu): arguments and launcher.
 #pragma once
 
+#include <algorithm>
+
 #include "query.cuh"
 
 namespace ckb {
@@ -10,6 +12,7 @@ struct FastArgs {
   query::QArgs q;       // tree / queries / outputs (ids, d2 [nq][k], max [nq])
   int kk;               // k (1 for FCP)
   bool fcp;             // FCP semantics (strict minimum, -1 beyond the cut-off)
+  int method;           // the named traversal (which tied candidates it visits)
   int *work;            // global chunk counter (zeroed before the launch)
   int *fb_count;        // fallback queue length (zeroed before the launch)
   int32_t *fb_list;     // fallback queue (query indices), capacity nq
@@ -20,16 +23,42 @@ struct FastArgs {
 
 }  // namespace fast
 
-// Launches the fast kernel for float trees with D = 2..4 and k <= 128
-// (register list up to k = 32, local-memory heap above).
-int run_fast(const fast::FastArgs &fa, int D, cudaStream_t st);
+// Whether a node's point can be read as one vector load (8 bytes for D = 2,
+// 16 for D = 3 and 4; for D = 3 with the split dim, if explicit, in the
+// fourth word): the records' stride, the point's place in them and the
+// array's address all have to be aligned.
+inline bool vector_points(const query::QArgs &a, int D)
+{
+  const int al = D == 2 ? 8 : 16;
+  if (a.stride % al || a.poff % al || reinterpret_cast<uintptr_t>(a.tree) % al) return false;
+  return D != 3 || a.doff < 0 || a.doff == a.poff + 12;
+}
+
+// Asks for no more shared memory per SM than the resident blocks' candidate
+// nodes take (kc words a thread): the driver's own choice leaves the stack
+// and the nodes less L1 (10M queries, k = 16: 132 KB, 10.85 ms; 82 KB,
+// 10.50 ms).
+template <class Kernel>
+inline void prefer_shared(Kernel *kernel, int threads, int block, int kc)
+{
+  const int bytes = threads * kc * 4 + (threads + block - 1) / block * 1024;
+  const int percent = std::min(100, (bytes * 100 + 228 * 1024 - 1) / (228 * 1024));
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, percent) !=
+      cudaSuccess)
+    cudaGetLastError();  // a preference only
+}
+
+// Launches the fast kernel for float (scalar 0) or int32 (scalar 1) trees
+// with D = 2..4 and k <= 128 (fast.cu).
+int run_fast(const fast::FastArgs &fa, int scalar, int D, cudaStream_t st);
+// the instantiations of one dimension (fast_d2.cu, fast_d3.cu, fast_d4.cu)
+template <int D> int run_fast_dim(const fast::FastArgs &fa, int scalar, cudaStream_t st);
+extern template int run_fast_dim<2>(const fast::FastArgs &, int, cudaStream_t);
+extern template int run_fast_dim<3>(const fast::FastArgs &, int, cudaStream_t);
+extern template int run_fast_dim<4>(const fast::FastArgs &, int, cudaStream_t);
 
 // The warp-cooperative traversal (packet.cu): float kNN, k = 2..32, no
 // forest, no device-side query count.
 int run_packet(const fast::FastArgs &fa, int D, cudaStream_t st);
-
-// The same for int32 trees (exact int64 distances), kNN with k = 2..128
-// (fast_int.cu).
-int run_fast_int(const fast::FastArgs &fa, int D, cudaStream_t st);
 
 }  // namespace ckb

@@ -309,11 +309,12 @@ __global__ void __launch_bounds__(128, 4) infer_kernel(const __nv_bfloat16 *__re
 // the network's instructions mostly fill issue slots the traversal leaves
 // idle.
 // ---------------------------------------------------------------------------
-template <int D, bool EXPL, bool VEC16, int KC>
-__global__ void __launch_bounds__(256, KC <= 17 ? 4 : 2)
-    knn_learned_kernel(fast::FastArgs fa, const __nv_bfloat16 *__restrict__ wbf,
+template <int D, bool EXPL, bool VEC, int KC>
+__global__ void __launch_bounds__(256, KC <= 17 ? 4 : 3)
+    knn_learned_kernel(const __grid_constant__ fast::FastArgs fa, const __nv_bfloat16 *__restrict__ wbf,
                        const float *__restrict__ dens, Norm nm)
 {
+  extern __shared__ uint32_t sh[];
   const int lane = threadIdx.x & 31;
   const int64_t nq = fa.q.nq;
   const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
@@ -330,42 +331,49 @@ __global__ void __launch_bounds__(256, KC <= 17 ? 4 : 2)
     __syncwarp();
     const float y = mlp_forward_warp(wbf, f);
     const float r = expf(__fmaf_rn(y, nm.tstd, nm.tmean));
-    if (live) fast::knn_fast_one<D, EXPL, VEC16, KC>(fa, i, myq, true, r);
+    if (live)
+      fast::knn_fast_one<0, D, EXPL, VEC, KC>(fa, myq, true, r, sh + threadIdx.x, blockDim.x);
   }
 }
 
-template <int D, bool EXPL, bool VEC16>
+template <int D, bool EXPL, bool VEC>
 int launch_learned(const fast::FastArgs &fa, const __nv_bfloat16 *wbf, const float *dens,
                    const Norm &nm, cudaStream_t st)
 {
   const int bs = 256;
   const unsigned grid = unsigned(std::max<int64_t>(1, div_up(fa.q.nq, bs)));
   const int slots = fa.kk + 1;
+#define CKB_LEARNED(KC_)                                                                   \
+  do {                                                                                     \
+    prefer_shared(knn_learned_kernel<D, EXPL, VEC, KC_>, KC_ <= 17 ? 1024 : 768, bs, KC_); \
+    knn_learned_kernel<D, EXPL, VEC, KC_><<<grid, bs, sizeof(uint32_t) * KC_ * bs, st>>>(  \
+        fa, wbf, dens, nm);                                                                \
+  } while (0)
   if (slots <= 5)
-    knn_learned_kernel<D, EXPL, VEC16, 5><<<grid, bs, 0, st>>>(fa, wbf, dens, nm);
+    CKB_LEARNED(5);
   else if (slots <= 9)
-    knn_learned_kernel<D, EXPL, VEC16, 9><<<grid, bs, 0, st>>>(fa, wbf, dens, nm);
+    CKB_LEARNED(9);
   else if (slots <= 17)
-    knn_learned_kernel<D, EXPL, VEC16, 17><<<grid, bs, 0, st>>>(fa, wbf, dens, nm);
+    CKB_LEARNED(17);
   else if (slots <= 33)
-    knn_learned_kernel<D, EXPL, VEC16, 33><<<grid, bs, 0, st>>>(fa, wbf, dens, nm);
+    CKB_LEARNED(33);
   else
     return CUKD_ERR_UNSUPPORTED;
+#undef CKB_LEARNED
   CKB_CHECK_LAUNCH();
   return CUKD_OK;
 }
 
 template <int D>
-int launch_learned_layout(const fast::FastArgs &fa, const Layout &L, const __nv_bfloat16 *wbf,
-                          const float *dens, const Norm &nm, cudaStream_t st)
+int launch_learned_layout(const fast::FastArgs &fa, const __nv_bfloat16 *wbf, const float *dens,
+                          const Norm &nm, cudaStream_t st)
 {
-  const bool expl = L.doff >= 0;
-  const bool vec16 = L.stride == 16 && L.poff == 0 && (!expl || L.doff == 12) && D <= 3;
-  if (expl)
-    return vec16 ? launch_learned<D, true, true>(fa, wbf, dens, nm, st)
-                 : launch_learned<D, true, false>(fa, wbf, dens, nm, st);
-  return vec16 ? launch_learned<D, false, true>(fa, wbf, dens, nm, st)
-               : launch_learned<D, false, false>(fa, wbf, dens, nm, st);
+  const bool vec = vector_points(fa.q, D);
+  if (fa.q.doff >= 0)
+    return vec ? launch_learned<D, true, true>(fa, wbf, dens, nm, st)
+               : launch_learned<D, true, false>(fa, wbf, dens, nm, st);
+  return vec ? launch_learned<D, false, true>(fa, wbf, dens, nm, st)
+             : launch_learned<D, false, false>(fa, wbf, dens, nm, st);
 }
 
 // (D, scalar) dispatch of the per-query model kernels
@@ -397,7 +405,6 @@ static void init_params(std::vector<float> &p, uint64_t seed, int D)
 
 }  // namespace learned
 
-int run_fast(const fast::FastArgs &fa, int D, cudaStream_t st);
 
 }  // namespace ckb
 
@@ -727,6 +734,7 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   fast::FastArgs fa = {};
   fa.q = a;
   fa.kk = p->k;
+  fa.method = p->method;
   fa.work = ctr;
   fa.fb_count = ctr + 1;
   fa.fb_list = fb1;
@@ -737,19 +745,18 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   if (isFloat && p->k <= 32 && !packet) {
     // pass 1: radii predicted and searched in one kernel
     const int D = L.D;
-    const int rc = D == 2 ? launch_learned_layout<2>(fa, L, m->d.wbf, m->d.dens, m->norm, st)
-                 : D == 3 ? launch_learned_layout<3>(fa, L, m->d.wbf, m->d.dens, m->norm, st)
-                          : launch_learned_layout<4>(fa, L, m->d.wbf, m->d.dens, m->norm, st);
+    const int rc = D == 2 ? launch_learned_layout<2>(fa, m->d.wbf, m->d.dens, m->norm, st)
+                 : D == 3 ? launch_learned_layout<3>(fa, m->d.wbf, m->d.dens, m->norm, st)
+                          : launch_learned_layout<4>(fa, m->d.wbf, m->d.dens, m->norm, st);
     CKB_TRY(rc);
   } else {
     // pass 1: the radii predicted for every query, then the seeded traversal
-    // (the local-memory heap for k > 32, or the integer kernel)
     float *radius = nullptr;
     CKB_TRY(arena.alloc(&radius, nq));
     CKB_TRY(infer_launch(m, d_queries, nq, radius, st));
     fa.radius = radius;
     CKB_TRY(packet ? run_packet(fa, L.D, st)
-                   : (isFloat ? run_fast(fa, L.D, st) : run_fast_int(fa, L.D, st)));
+                   : run_fast(fa, L.scalar, L.D, st));
   }
   // pass 2: plain unbounded traversal of the queries pass 1 could not answer
   fast::FastArgs fb = fa;
@@ -759,7 +766,7 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   fb.q.count_ptr = ctr + 1;
   fb.fb_count = ctr + 2;
   fb.fb_list = fb2;
-  CKB_TRY(isFloat ? run_fast(fb, L.D, st) : run_fast_int(fb, L.D, st));
+  CKB_TRY(run_fast(fb, L.scalar, L.D, st));
   // pass 3: boundary ties in the reference's visiting order
   query::QArgs c = a;
   c.order = fb2;

@@ -24,6 +24,37 @@ namespace fast {
 
 using query::QArgs;
 
+// Far-child stack entries hold the node and, per dimension, the squared
+// offset from the query to the closest point of the node's box, truncated
+// to bf16 (the top 16 bits of the float): 12 bytes for D = 3 or 4, 8 for
+// D = 2, instead of the closest point plus its distance (20 bytes).
+// Truncation rounds toward zero, so a popped box's distance -- the sum of
+// its truncated offsets -- never exceeds the exact corner distance: culling
+// only becomes more permissive, and the answer cannot change.
+template <int D> struct PackedOffsets {
+  static constexpr int W = (D + 1) / 2;
+  uint32_t w[W];
+};
+template <int D>
+__device__ __forceinline__ PackedOffsets<D> pack_offsets(const float (&o)[D])
+{
+  PackedOffsets<D> p;
+#pragma unroll
+  for (int j = 0; j < PackedOffsets<D>::W; j++) {
+    const uint32_t lo = __float_as_uint(o[2 * j]) >> 16;
+    const uint32_t hi = 2 * j + 1 < D ? (__float_as_uint(o[2 * j + 1]) & 0xffff0000u) : 0u;
+    p.w[j] = hi | lo;
+  }
+  return p;
+}
+template <int D>
+__device__ __forceinline__ void unpack_offsets(const uint32_t *w, float (&o)[D])
+{
+#pragma unroll
+  for (int d = 0; d < D; d++)
+    o[d] = __uint_as_float((d & 1) ? (w[d >> 1] & 0xffff0000u) : (w[d >> 1] << 16));
+}
+
 template <int D, bool EXPL, bool VEC16, int KC>
 __global__ void __launch_bounds__(128, 4) knn_packet_kernel(FastArgs fa)
 {
@@ -270,7 +301,7 @@ int packet_layout(const FastArgs &fa, cudaStream_t st)
 {
   const QArgs &a = fa.q;
   const bool expl = a.doff >= 0;
-  const bool vec16 = a.stride == 16 && a.poff == 0 && (!expl || a.doff == 12) && D <= 3;
+  const bool vec16 = vec16_records(a.tree, a.stride, a.poff, a.doff, D);
   if (expl) return vec16 ? packet_kc<D, true, true>(fa, st) : packet_kc<D, true, false>(fa, st);
   return vec16 ? packet_kc<D, false, true>(fa, st) : packet_kc<D, false, false>(fa, st);
 }

@@ -108,7 +108,7 @@ int run_tree_path(const QArgs &a, int scalar, int D, int levels, uint32_t *codes
                   cudaStream_t st)
 {
   const bool expl = a.doff >= 0;
-  const bool vec16 = a.stride == 16 && a.poff == 0 && (!expl || a.doff == 12) && D <= 3;
+  const bool vec16 = vec16_records(a.tree, a.stride, a.poff, a.doff, D);
 #define CKB_TP(SC_, D_)                                                                   \
   if (scalar == SC_ && D == D_) {                                                         \
     if (expl) return vec16 ? launch_tree_path<SC_, D_, true, true>(a, levels, codes, vals, st) \
@@ -163,7 +163,7 @@ template <int SC, int D>
 int dispatch_layout(const QArgs &a, int method, int kind, cudaStream_t st)
 {
   const bool expl = a.doff >= 0;
-  const bool vec16 = a.stride == 16 && a.poff == 0 && (!expl || a.doff == 12) && D <= 3;
+  const bool vec16 = vec16_records(a.tree, a.stride, a.poff, a.doff, D);
   if (expl) {
     if (vec16) return dispatch_method<SC, D, true, true>(a, method, kind, st);
     return dispatch_method<SC, D, true, false>(a, method, kind, st);
@@ -270,8 +270,9 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
   if (fastOk) {
     fast::FastArgs fa = {};
     fa.q = a;
-    fa.kk = knn ? p->k : 1;
+    fa.kk = a.k;
     fa.fcp = !knn;
+    fa.method = p->method;
     int *ctr = nullptr;
     CKB_TRY(arena.alloc(&ctr, 2));
     CKB_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(int), st));
@@ -280,8 +281,7 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     CKB_TRY(arena.alloc(&fa.fb_list, nq));
     const bool packet = (p->flags & CUKD_QUERY_WARP_PACKET) && L.scalar == CUKD_FLOAT32 &&
                         knn && p->k <= 32;
-    CKB_TRY(packet ? run_packet(fa, L.D, st)
-                   : (L.scalar == CUKD_FLOAT32 ? run_fast(fa, L.D, st) : run_fast_int(fa, L.D, st)));
+    CKB_TRY(packet ? run_packet(fa, L.D, st) : run_fast(fa, L.scalar, L.D, st));
     if (p->d_reordered_count)
       CKB_CUDA(cudaMemcpyAsync(p->d_reordered_count, fa.fb_count, sizeof(int),
                                cudaMemcpyDeviceToDevice, st));

@@ -211,7 +211,7 @@ int dispatch(const QArgs &a, int k, int init, unsigned long long *lists, uint32_
              cudaStream_t st)
 {
   const bool expl = a.doff >= 0;
-  const bool vec16 = a.stride == 16 && a.poff == 0 && (!expl || a.doff == 12) && D <= 3;
+  const bool vec16 = vec16_records(a.tree, a.stride, a.poff, a.doff, D);
   if (expl) {
     if (vec16) return launch<D, true, true>(a, k, init, lists, off, st);
     return launch<D, true, false>(a, k, init, lists, off, st);

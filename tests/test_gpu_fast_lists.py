@@ -1,0 +1,68 @@
+"""The fast kNN kernel (fast_one.cuh) against the reference-order kernels at
+the sizes where it can go wrong: trees around the home subtree's size and a
+partly filled last level, lists at and around each compiled capacity, cut-offs
+that leave lists unfilled, records that can and cannot be read as vectors,
+tie-heavy and duplicate points.  Bit-exact: the reference-order kernels are
+pinned to the oracle in test_gpu_query.py.
+"""
+import math
+
+import pytest
+import torch
+
+import cudakdtree_b200 as ck
+from tests.helpers import make_points, make_queries
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(tree, q, k, method, lay, wb, **kw):
+    a = ck.knn(tree, q, k, method, layout=lay, world_bounds=wb, with_max=True, **kw)
+    b = ck.knn(tree, q, k, method, layout=lay, world_bounds=wb, with_max=True,
+               reference_order=True, **kw)
+    for x, y in zip(a, b):
+        assert torch.equal(x.view(torch.int32), y.view(torch.int32))
+
+
+@pytest.mark.parametrize("k", [2, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 127, 128])
+@pytest.mark.parametrize("scalar", ["float32", "int32"])
+@pytest.mark.parametrize("kind", ["uniform", "tie", "same"])
+def test_tree_sizes_and_list_capacities(k, scalar, kind):
+    q = torch.from_numpy(make_queries(333, 3, kind, scalar=scalar, seed=2)).cuda()
+    for n in (1, 2, k - 1, k, k + 1, 2 * k, 62, 63, 64, 127, 255, 256, 300, 1023, 5000):
+        tree = torch.from_numpy(make_points(n, 3, kind, scalar=scalar, seed=n)).cuda()
+        wb = ck.build_tree(tree)
+        _check(tree, q, k, ["stack_based", "stack_free", "cct"][n % 3], None, wb)
+
+
+@pytest.mark.parametrize("D", [2, 3, 4])
+@pytest.mark.parametrize("scalar", ["float32", "int32"])
+@pytest.mark.parametrize("k,cutoff", [(2, 0.03), (16, 0.1), (40, 0.2)])
+def test_cutoffs_and_record_layouts(D, scalar, k, cutoff):
+    n = 3001
+    pts = torch.from_numpy(make_points(n, D, "uniform", scalar=scalar, seed=5)).cuda()
+    q = torch.from_numpy(make_queries(777, D, "uniform", scalar=scalar, seed=6)).cuda()
+    kw = {"cutoff": cutoff} if scalar == "float32" else {"cutoff_d2": int((2000 * cutoff) ** 2)}
+    for stride, poff, doff, shift in ((4 * D, 0, -1, 0), (4 * D + 4, 0, 4 * D, 0),
+                                      (32, 16, -1, 0), (32, 0, 28, 4), (24, 4, 0, 0)):
+        lay = ck.layout_for(scalar, D, stride=stride, point_offset=poff, dim_offset=doff,
+                            dim_shift=shift, dim_bits=32 - shift)
+        words = torch.zeros(n * stride // 4 + 1, dtype=torch.int32, device="cuda")
+        for first in (0, 1):  # an array that starts 4 bytes off a 16-byte boundary
+            tree = words[first:first + n * stride // 4]
+            tree.view(n, -1)[:, poff // 4:poff // 4 + D] = pts.view(torch.int32)
+            wb = ck.build_tree(tree, layout=lay)
+            for method in ("stack_free", "cct"):
+                _check(tree, q, k, method, lay, wb)
+                _check(tree, q, k, method, lay, wb, **kw)
+
+
+@pytest.mark.parametrize("scale", [1e-25, 1e-12, 1e12, 1e18])
+def test_extreme_scales(scale):
+    """Bounds too small to scale stack entries by, and near the float range."""
+    pts = torch.from_numpy(make_points(5000, 3, "gmm", seed=7)).cuda() * scale
+    q = torch.from_numpy(make_queries(500, 3, "gmm", seed=8)).cuda() * scale
+    wb = ck.build_tree(pts)
+    for k in (3, 16, 64):
+        _check(pts, q, k, "stack_based", None, wb)
+        _check(pts, q, k, "cct", None, wb, cutoff=math.inf, morton=False)
