@@ -420,7 +420,6 @@ static int query_impl(cukd_batch_plan_s *p, const float *pts, const float *bound
     fa.fcp = false;
     fa.method = p->params.method;
     CKB_CUDA(cudaMemsetAsync(p->ctr, 0, 2 * sizeof(int), st));
-    fa.work = p->ctr;
     fa.fb_count = p->ctr + 1;
     fa.fb_list = p->fb_list;
     CKB_TRY(run_fast(fa, CUKD_FLOAT32, D, st));

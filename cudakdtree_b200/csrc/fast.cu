@@ -44,6 +44,11 @@
 #include "fast.cuh"
 
 namespace ckb {
+namespace fast {
+template <int SC> int run_warp_scalar(const WarpArgs &wa, int D, cudaStream_t st);
+extern template int run_warp_scalar<0>(const WarpArgs &, int, cudaStream_t);
+extern template int run_warp_scalar<1>(const WarpArgs &, int, cudaStream_t);
+}  // namespace fast
 
 int run_fast(const fast::FastArgs &fa, int scalar, int D, cudaStream_t st)
 {
@@ -51,6 +56,12 @@ int run_fast(const fast::FastArgs &fa, int scalar, int D, cudaStream_t st)
   if (D == 3) return run_fast_dim<3>(fa, scalar, st);
   if (D == 4) return run_fast_dim<4>(fa, scalar, st);
   return CUKD_ERR_UNSUPPORTED;
+}
+
+int run_warp(const fast::WarpArgs &wa, int scalar, int D, cudaStream_t st)
+{
+  return scalar == CUKD_FLOAT32 ? fast::run_warp_scalar<0>(wa, D, st)
+                                : fast::run_warp_scalar<1>(wa, D, st);
 }
 
 }  // namespace ckb

@@ -13,12 +13,19 @@ struct FastArgs {
   int kk;               // k (1 for FCP)
   bool fcp;             // FCP semantics (strict minimum, -1 beyond the cut-off)
   int method;           // the named traversal (which tied candidates it visits)
-  int *work;            // global chunk counter (zeroed before the launch)
   int *fb_count;        // fallback queue length (zeroed before the launch)
   int32_t *fb_list;     // fallback queue (query indices), capacity nq
   const float *radius;  // optional per-query initial cull radius (before scaling)
   int32_t *status;      // optional per-query outcome: 0 answered, 1 queued
   float radius_scale;   // multiplies `radius`
+  int queue_min;        // with q.count_ptr: a queue of at most this many is left alone
+};
+
+// the warp-per-query kernel's arguments (warp.cuh)
+struct WarpArgs {
+  FastArgs f;
+  int queue_limit;  // with f.q.count_ptr: a longer queue is handed over, or left alone
+  bool hand_over;   // copy such a queue to f.fb_list
 };
 
 }  // namespace fast
@@ -56,6 +63,23 @@ template <int D> int run_fast_dim(const fast::FastArgs &fa, int scalar, cudaStre
 extern template int run_fast_dim<2>(const fast::FastArgs &, int, cudaStream_t);
 extern template int run_fast_dim<3>(const fast::FastArgs &, int, cudaStream_t);
 extern template int run_fast_dim<4>(const fast::FastArgs &, int, cudaStream_t);
+
+// The same answers with a warp per query (warp.cuh): lower latency, about a
+// fifth of the throughput.  All of q.nq, or a device-side queue.
+int run_warp(const fast::WarpArgs &wa, int scalar, int D, cudaStream_t st);
+
+// Calls of at most this many queries are answered a warp each; the line
+// lies where the two kernels take the same time.  Whole calls, us, thread /
+// warp per query (B200, uniform float3, 100K points): k = 8, 1000 queries
+// 157 / 41, 16384 175 / 117, 32768 181 / 200; k = 32, 16384 257 / 206; k = 64,
+// 8192 367 / 295, 16384 361 / 530; int3, 1M points, k = 16, 8192 146 / 122,
+// 16384 146 / 198.
+inline int64_t warp_queries(int scalar, int k)
+{
+  return scalar == CUKD_FLOAT32 && k <= 32 ? 16384 : 8192;
+}
+// and queued queries, of which the host does not know how many there are
+constexpr int kWarpQueue = 8192;
 
 // The warp-cooperative traversal (packet.cu): float kNN, k = 2..32, no
 // forest, no device-side query count.

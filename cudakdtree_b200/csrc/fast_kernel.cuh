@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(fast_threads(KC), fast_blocks(KC))
 {
   extern __shared__ uint32_t sh[];
   const int64_t limit = fa.q.count_ptr ? int64_t(*fa.q.count_ptr) : fa.q.nq;
+  if (fa.q.count_ptr && limit <= fa.queue_min) return;
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < limit;
        i += int64_t(gridDim.x) * blockDim.x) {
     const int64_t myq = fa.q.order ? int64_t(fa.q.order[i]) : i;

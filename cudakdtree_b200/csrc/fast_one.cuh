@@ -108,6 +108,13 @@ struct Nodes {
     point(node, p);
     return dim_of(node);
   }
+  // the same for a node whose level is known
+  __device__ __forceinline__ int load_at(int node, int lvl, T (&p)[D]) const
+  {
+    if (EXPL) return load(node, p);
+    point(node, p);
+    return lvl % D;
+  }
   __device__ __forceinline__ void point(int node, T (&p)[D]) const
   {
     const uint8_t *c = tree + int64_t(node) * stride + poff;

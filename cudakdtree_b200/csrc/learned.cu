@@ -735,7 +735,6 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   fa.q = a;
   fa.kk = p->k;
   fa.method = p->method;
-  fa.work = ctr;
   fa.fb_count = ctr + 1;
   fa.fb_list = fb1;
   fa.radius_scale = radius_scale;
@@ -758,7 +757,8 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
     CKB_TRY(packet ? run_packet(fa, L.D, st)
                    : run_fast(fa, L.scalar, L.D, st));
   }
-  // pass 2: plain unbounded traversal of the queries pass 1 could not answer
+  // pass 2: unbounded search of the queries pass 1 could not answer, a warp
+  // each while they are few
   fast::FastArgs fb = fa;
   fb.radius = nullptr;
   fb.status = nullptr;
@@ -766,6 +766,13 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   fb.q.count_ptr = ctr + 1;
   fb.fb_count = ctr + 2;
   fb.fb_list = fb2;
+  fb.queue_min = 0;
+  if (!d_visits) {
+    fast::WarpArgs wa = {};
+    wa.f = fb;
+    wa.queue_limit = fb.queue_min = kWarpQueue;
+    CKB_TRY(run_warp(wa, L.scalar, L.D, st));
+  }
   CKB_TRY(run_fast(fb, L.scalar, L.D, st));
   // pass 3: boundary ties in the reference's visiting order
   query::QArgs c = a;

@@ -238,8 +238,36 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
   a.visits = visits;
   a.block_size = p->block_size;
   TempArena arena(st, mem);
-  // query orders (tree path, Morton) and the fast path: up to 4 dims
+  // query orders (tree path, Morton) and the fast paths: up to 4 dims
   const bool narrow = L.D <= kMaxFastDims;
+  const bool exactOk = !visits && !a.heap_order && !(p->flags & CUKD_QUERY_REFERENCE_ORDER) &&
+                       a.k <= 128 && narrow;
+  // few queries: a warp each (in any order, so without sorting them), and
+  // what it queues by the named traversal.  A stack-free FCP or k = 1 with
+  // eps may return a point that is not the closest: only its own traversal
+  // says which.
+  if (exactOk && nq <= warp_queries(L.scalar, a.k) &&
+      !(p->method == CUKD_STACK_FREE && p->eps != 0.f && a.k == 1)) {
+    fast::WarpArgs wa = {};
+    fast::FastArgs &fa = wa.f;
+    fa.q = a;
+    fa.kk = a.k;
+    fa.fcp = !knn;
+    fa.method = p->method;
+    int *queue = nullptr;  // its length, then the queries
+    CKB_TRY(arena.alloc(&queue, nq + 1));
+    CKB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), st));
+    fa.fb_count = queue;
+    fa.fb_list = queue + 1;
+    CKB_TRY(run_warp(wa, L.scalar, L.D, st));
+    if (p->d_reordered_count)
+      CKB_CUDA(cudaMemcpyAsync(p->d_reordered_count, fa.fb_count, sizeof(int),
+                               cudaMemcpyDeviceToDevice, st));
+    QArgs b = a;
+    b.order = fa.fb_list;
+    b.count_ptr = fa.fb_count;
+    return run_query(b, L.scalar, L.D, p->method, kind, st);
+  }
   if ((p->flags & CUKD_QUERY_TREE_ORDER) && nq > 1 && n > 0 && narrow) {
     uint32_t *codes = nullptr, *codes2 = nullptr, *vals = nullptr, *vals2 = nullptr;
     CKB_TRY(arena.alloc(&codes, nq));
@@ -261,33 +289,40 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     a.order = perm;
   }
   // fast exact path (see fast.cu): any visiting order, boundary-tie check,
-  // reference-order re-run of the queued queries
-  const bool fastOk = !visits && !a.heap_order && !(p->flags & CUKD_QUERY_REFERENCE_ORDER) &&
-                      knn && p->k >= 2 && p->k <= 128 && n < (int64_t(1) << 31) - 1 && narrow;
-  // (FCP and k = 1 stay on the reference traversals: with a single
-  // candidate the split-plane bound is already cheap and the corner
-  // bookkeeping does not pay for itself)
-  if (fastOk) {
+  // the queued queries a warp each, what that leaves in the reference order.
+  // (FCP and k = 1 stay on the reference traversals: with a single candidate
+  // the split-plane bound is already cheap and the corner bookkeeping does
+  // not pay for itself)
+  if (exactOk && knn && p->k >= 2) {
+    fast::WarpArgs wa = {};
     fast::FastArgs fa = {};
     fa.q = a;
     fa.kk = a.k;
-    fa.fcp = !knn;
     fa.method = p->method;
     int *ctr = nullptr;
+    int32_t *lists = nullptr;
     CKB_TRY(arena.alloc(&ctr, 2));
     CKB_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(int), st));
-    fa.work = ctr;
-    fa.fb_count = ctr + 1;
-    CKB_TRY(arena.alloc(&fa.fb_list, nq));
+    CKB_TRY(arena.alloc(&lists, 2 * nq));
+    fa.fb_count = ctr;
+    fa.fb_list = lists;
     const bool packet = (p->flags & CUKD_QUERY_WARP_PACKET) && L.scalar == CUKD_FLOAT32 &&
-                        knn && p->k <= 32;
+                        p->k <= 32;
     CKB_TRY(packet ? run_packet(fa, L.D, st) : run_fast(fa, L.scalar, L.D, st));
+    wa.f = fa;
+    wa.f.q.order = fa.fb_list;
+    wa.f.q.count_ptr = fa.fb_count;
+    wa.f.fb_count = ctr + 1;
+    wa.f.fb_list = lists + nq;
+    wa.queue_limit = kWarpQueue;
+    wa.hand_over = true;
+    CKB_TRY(run_warp(wa, L.scalar, L.D, st));
     if (p->d_reordered_count)
-      CKB_CUDA(cudaMemcpyAsync(p->d_reordered_count, fa.fb_count, sizeof(int),
+      CKB_CUDA(cudaMemcpyAsync(p->d_reordered_count, ctr + 1, sizeof(int),
                                cudaMemcpyDeviceToDevice, st));
     QArgs b = a;
-    b.order = fa.fb_list;
-    b.count_ptr = fa.fb_count;
+    b.order = wa.f.fb_list;
+    b.count_ptr = wa.f.fb_count;
     return run_query(b, L.scalar, L.D, p->method, kind, st);
   }
   return run_query(a, L.scalar, L.D, p->method, kind, st);
