@@ -730,7 +730,7 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   CKB_CUDA(cudaMemsetAsync(ctr, 0, 4 * sizeof(int), st));
   int32_t *fb1 = nullptr, *fb2 = nullptr;
   CKB_TRY(arena.alloc(&fb1, nq));
-  CKB_TRY(arena.alloc(&fb2, nq));
+  CKB_TRY(arena.alloc(&fb2, 2 * nq));
   fast::FastArgs fa = {};
   fa.q = a;
   fa.kk = p->k;
@@ -758,22 +758,34 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
                    : run_fast(fa, L.scalar, L.D, st));
   }
   // pass 2: unbounded search of the queries pass 1 could not answer, a warp
-  // each while they are few
+  // each while they are few (32768: of queries far from every point, which
+  // are most of them, a warp each takes a third of the time); boundary ties
+  // of the other kernel a warp each, too
   fast::FastArgs fb = fa;
   fb.radius = nullptr;
   fb.status = nullptr;
   fb.q.order = fb1;
   fb.q.count_ptr = ctr + 1;
-  fb.fb_count = ctr + 2;
-  fb.fb_list = fb2;
-  fb.queue_min = 0;
+  fb.fb_count = ctr + 3;
+  fb.fb_list = fb2 + nq;
+  fast::WarpArgs wa = {};
   if (!d_visits) {
-    fast::WarpArgs wa = {};
     wa.f = fb;
-    wa.queue_limit = fb.queue_min = kWarpQueue;
+    wa.f.fb_count = ctr + 2;
+    wa.f.fb_list = fb2;
+    wa.queue_limit = fb.queue_min = 32768;
     CKB_TRY(run_warp(wa, L.scalar, L.D, st));
   }
   CKB_TRY(run_fast(fb, L.scalar, L.D, st));
+  wa.f = fb;
+  wa.f.q.visits = nullptr;
+  wa.f.q.order = fb.fb_list;
+  wa.f.q.count_ptr = fb.fb_count;
+  wa.f.fb_count = ctr + 2;
+  wa.f.fb_list = fb2;
+  wa.queue_limit = kWarpQueue;
+  wa.hand_over = true;
+  CKB_TRY(run_warp(wa, L.scalar, L.D, st));
   // pass 3: boundary ties in the reference's visiting order
   query::QArgs c = a;
   c.order = fb2;

@@ -109,10 +109,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     limit = *a.count_ptr;
     if (limit > wa.queue_limit) {
       if (!wa.hand_over) return;
+      // (behind what is queued there already: each block takes its share)
       for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < limit;
            i += int64_t(gridDim.x) * blockDim.x)
-        fa.fb_list[i] = a.order[i];
-      if (blockIdx.x == 0 && threadIdx.x == 0) *fa.fb_count = int(limit);
+        fa.fb_list[atomicAdd(fa.fb_count, 1)] = a.order[i];
       return;
     }
   }
