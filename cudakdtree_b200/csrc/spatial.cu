@@ -19,17 +19,30 @@
 // reference's int32 order-preserving float encoding (:177-192).
 //
 // Data layout.  Prims are kept in segments, one per open node, in prim-id
-// order; a pass stably partitions each split node's segment into its two
-// children's segments (two device-wide scans), so every node's prims stay
-// contiguous and ordered.  One device->host read per pass decides whether
-// another pass is needed (the reference reads the node count every pass).
+// order; a level stably partitions each split node's segment into its two
+// children's segments, so every node's prims stay contiguous and ordered.
+//
+// Two phases.  Nodes of more than kSub prims are split level by level by
+// all CTAs (three launches a level: side bits with their prefix sums, the
+// nodes' children, the move with the children's boxes); what is left at
+// kSub prims or fewer becomes the root of a subtree that one CTA finishes in
+// shared memory.  Neither phase numbers nodes: a split node is stored under
+// the boundary between its children's prims, a leaf under its first prim,
+// which are unique, and in which nodes of one level stand in the order of
+// their numbers.  Sorting those places by level (stably) numbers the nodes.
+// The host reads back twice, plus once per four levels beyond the expected.
+//
+// Before, every level of the tree (27 for 1M mixture points) ran twelve
+// launches and a device->host read of its split count: 2.6 ms for 1M points
+// (B200), of which the kernels took 2.1 ms, against 1.0 ms now (20 levels
+// 0.63 ms, bound by their launches and scattered moves; subtrees 0.18 ms).
 #include <algorithm>
 #include <cfloat>
-#include <vector>
 
 #include "common.cuh"
 #include "query.cuh"
 #include "scan.cuh"
+#include "sort.cuh"
 
 namespace ckb {
 namespace spatial {
@@ -60,20 +73,41 @@ __host__ __device__ inline float dec(int32_t b)
 #endif
 }
 
+constexpr uint32_t kSub = 1024;       // prims of a subtree that one CTA finishes
+constexpr uint32_t kDone = 0xffffffffu;  // position not in an open node of the level phase
+constexpr int kSideTile = 1024;  // positions of a CTA of side_kernel
+constexpr int kSideWords = kSideTile / 8 / 32;  // per warp
+
+struct SubRoot {
+  uint32_t begin, count, level;
+  uint32_t link;    // parent's boundary * 2 + (this is its left child); kDone: none
+  uint32_t parity;  // buffer that holds its prims
+};
+
+struct BuildState {  // device-side counters
+  uint32_t open[2];  // open nodes of the level phase, by parity of the level
+  uint32_t subRoots, leaves, maxLevel, ticket;
+};
+
 struct BuildBufs {
-  // per node (capacity 2n+2)
-  uint32_t *count, *segBegin;
-  int32_t *lo, *hi;  // [node][D], encoded
-  int32_t *sdim;     // split dim of open nodes (-1 degenerate)
-  float *spos;
-  Node *out;
-  // per open node of the current pass
-  uint32_t *isSplit, *splitRank;
-  // per prim position
+  BuildState *st;
+  // open nodes of the level phase, by parity
+  uint32_t *begin[2], *count[2], *link[2];
+  int32_t *lo[2], *hi[2];  // [node][D], encoded
+  uint4 *move;             // per open node: first position, left prims before it,
+                           // left prims, (unused)
+  uint2 *codes;            // its children's open nodes of the next level, or kDone
+  // side bits of a level's prims: words, their prefix within a tile, tile sums
+  uint32_t *bits, *wordPre, *tileBase;
+  SubRoot *roots;
+  // the tree by place: splits under their boundary, leaves under their first
+  // prim; key[2 * first] / key[2 * boundary - 1] holds the node's level
+  uint32_t *key, *splitChild, *leaf;  // leaf: prim count, buffer in bit 31
+  float *splitPos;
+  uint8_t *splitDim;
+  // per prim position, by parity
   uint32_t *prim[2], *nodeOf[2];
   float *coord[2][4];  // the prim's coordinates, moved with it (SoA per dim)
-  uint32_t *fl;        // goes-left flags -> exclusive scan
-  uint32_t *total;    // scan totals / pass counters [4]
   const uint8_t *data;
   int stride, poff;
 };
@@ -187,189 +221,492 @@ __global__ void init_kernel(BuildBufs b, int64_t n)
 #pragma unroll
     for (int d = 0; d < D; d++) p[d] = 0.f;
   }
-  block_grow<D>(b.lo, b.hi, 0, valid, p);
+  block_grow<D>(b.lo[0], b.hi[0], 0, valid, p);
 }
 
-template <int D>
-__global__ void root_setup_kernel(BuildBufs b, int64_t n)
+__device__ inline void note_leaf(const BuildBufs &b, uint32_t begin, uint32_t count,
+                                 uint32_t level, uint32_t parity, uint32_t link)
 {
-  if (threadIdx.x != 0) return;
-  b.count[0] = uint32_t(n);
-  b.segBegin[0] = 0;
-  // node 1: the reference's empty dummy (initState, :276-290)
-  b.out[1].pos = 0.f;
-  b.out[1].offset = 0;
-  b.out[1].count = 0;
-  b.out[1].dim = 0;
+  b.key[2 * size_t(begin)] = level;
+  b.leaf[begin] = count | (parity << 31);
+  if (link != kDone && (link & 1)) b.splitChild[link >> 1] = 2 * begin;
+}
+__device__ inline void note_split(const BuildBufs &b, uint32_t boundary, int dim, float pos,
+                                  uint32_t level, uint32_t link)
+{
+  b.key[2 * size_t(boundary) - 1] = level;
+  b.splitPos[boundary] = pos;
+  b.splitDim[boundary] = uint8_t(dim < 0 ? 0 : dim);
+  if (link != kDone && (link & 1)) b.splitChild[link >> 1] = 2 * boundary - 1;
 }
 
-// selectSplits (:316-396) for the open nodes [pb, pe)
-template <int D>
-__global__ void decide_kernel(BuildBufs b, uint32_t pb, uint32_t pe, int threshold)
+// the root: a leaf, a subtree, or the first open node
+__global__ void root_kernel(BuildBufs b, uint32_t n, uint32_t threshold)
 {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= pe - pb) return;
-  const uint32_t node = pb + t;
-  const uint32_t cnt = b.count[node];
-  if (int64_t(cnt) <= threshold) {
-    b.isSplit[t] = 0;
-    b.out[node].offset = 0;  // leaves with prims get theirs at the end
-    b.out[node].count = uint16_t(cnt);
-    b.out[node].dim = 0;
-    b.out[node].pos = 0.f;
-    return;
+  BuildState s = {};
+  if (n <= threshold) {
+    note_leaf(b, 0, n, 0, 0, kDone);
+    s.leaves = 1;
+  } else if (n <= kSub) {
+    b.roots[0] = SubRoot{0, n, 0, kDone, 0};
+    s.subRoots = 1;
+  } else {
+    b.begin[0][0] = 0;
+    b.count[0][0] = n;
+    b.link[0][0] = kDone;
+    s.open[0] = 1;
   }
-  float widestWidth = 0.f;
-  int widestDim = -1;
+  *b.st = s;
+}
+
+// selectSplits (:316-396): the widest extent's centre; dim -1: degenerate
+template <int D>
+__device__ inline int decide(const int32_t *lo, const int32_t *hi, float *pos)
+{
+  float widestWidth = 0.f, at = 0.f;
+  int dim = -1;
+#pragma unroll
   for (int d = 0; d < D; d++) {
-    const float width = __fsub_rn(dec(b.hi[int64_t(node) * D + d]), dec(b.lo[int64_t(node) * D + d]));
+    const float l = dec(lo[d]), h = dec(hi[d]);
+    const float width = __fsub_rn(h, l);
     if (width <= widestWidth) continue;
     widestWidth = width;
-    widestDim = d;
+    dim = d;
+    at = __fmul_rn(0.5f, __fadd_rn(l, h));
+    if (at == l || at == h) dim = -2 - d;  // rounds onto the box
   }
-  float pos = 0.f;
-  if (widestDim >= 0) {
-    const float l = dec(b.lo[int64_t(node) * D + widestDim]);
-    const float h = dec(b.hi[int64_t(node) * D + widestDim]);
-    pos = __fmul_rn(0.5f, __fadd_rn(l, h));
-    if (pos == l || pos == h) widestDim = -1;
+  if (dim < 0) {
+    dim = -1;
+    at = dec(lo[0]);
   }
-  if (widestDim < 0) pos = dec(b.lo[int64_t(node) * D + 0]);
-  b.sdim[node] = widestDim;
-  b.spos[node] = pos;
-  b.isSplit[t] = 1;
+  *pos = at;
+  return dim;
 }
 
-// children ids (parent order), split node records, empty child boxes
-template <int D>
-__global__ void children_kernel(BuildBufs b, uint32_t pb, uint32_t pe, uint32_t childBase)
+// Left-side prims at positions below p (the level's side bits).
+__device__ inline uint32_t left_before(const BuildBufs &b, uint32_t p)
 {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= pe - pb || !b.isSplit[t]) return;
-  const uint32_t node = pb + t;
-  const uint32_t first = childBase + 2 * b.splitRank[t];
-  const int dim = b.sdim[node];
-  b.out[node].offset = first;
-  b.out[node].count = 0;
-  b.out[node].dim = int16_t(dim < 0 ? 0 : dim);
-  b.out[node].pos = b.spos[node];
-  for (int s = 0; s < 2; s++) {
-    for (int d = 0; d < D; d++) {
-      b.lo[int64_t(first + s) * D + d] = enc(+FLT_MAX);
-      b.hi[int64_t(first + s) * D + d] = enc(-FLT_MAX);
+  const uint32_t t = b.tileBase[p / kSideTile];
+  if ((p & (kSideTile - 1)) == 0) return t;
+  const uint32_t w = p >> 5;
+  return t + b.wordPre[w] + __popc(b.bits[w] & ((1u << (p & 31)) - 1u));
+}
+
+// updatePrims (:398-436): a bit per prim of an open node that goes left, the
+// bits' prefix sums within kSideTile-prim tiles, and (the last CTA) over tiles.
+// Every prim decides its node's split itself: the box is in L1, and a launch
+// of its own would cost more.
+template <int D>
+__global__ void __launch_bounds__(256) side_kernel(BuildBufs b, int64_t n, int par, int tiles)
+{
+  __shared__ uint32_t warpSum[8];
+  __shared__ bool last;
+  // (also without open nodes: the next level must find none either)
+  if (blockIdx.x == 0 && threadIdx.x == 0) b.st->open[par ^ 1] = 0;
+  if (b.st->open[par] == 0) return;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t base = int64_t(blockIdx.x) * kSideTile + wid * (32 * kSideWords);
+  uint32_t word = 0;
+#pragma unroll
+  for (int j = 0; j < kSideWords; j++) {
+    const int64_t p = base + 32 * j + lane;
+    bool left = false;
+    if (p < n) {
+      const uint32_t node = b.nodeOf[par][p];
+      if (node != kDone) {
+        float pos;
+        const int dim = decide<D>(b.lo[par] + int64_t(node) * D, b.hi[par] + int64_t(node) * D,
+                                  &pos);
+        left = dim < 0 ? ((uint32_t(p) - b.begin[par][node]) & 1u) == 0
+                       : !(b.coord[par][dim][p] >= pos);
+      }
+    }
+    const uint32_t w = __ballot_sync(0xffffffffu, left);
+    if (lane == j) word = w;
+  }
+  const uint32_t c = lane < kSideWords ? __popc(word) : 0;
+  uint32_t incl = c;
+#pragma unroll
+  for (int o = 1; o < kSideWords; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == kSideWords - 1) warpSum[wid] = incl;
+  __syncthreads();
+  uint32_t before = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < 8; w++) {
+    before += w < wid ? warpSum[w] : 0;
+    total += warpSum[w];
+  }
+  if (lane < kSideWords) {
+    b.bits[(base >> 5) + lane] = word;
+    b.wordPre[(base >> 5) + lane] = before + incl - c;
+  }
+  if (threadIdx.x == 0) {
+    b.tileBase[blockIdx.x] = total;
+    __threadfence();
+    last = atomicAdd(&b.st->ticket, 1u) + 1 == gridDim.x;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // exclusive scan of the tile sums, [tiles] = their total
+  uint32_t carry = 0;
+  for (int off = 0; off < tiles; off += 1024) {
+    uint32_t v[4], s = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int i = off + threadIdx.x * 4 + j;
+      v[j] = i < tiles ? __ldcg(b.tileBase + i) : 0u;
+      s += v[j];
+    }
+    uint32_t in = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, in, o);
+      if (lane >= o) in += t;
+    }
+    __syncthreads();
+    if (lane == 31) warpSum[wid] = in;
+    __syncthreads();
+    uint32_t run = carry + in - s;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      run += w < wid ? warpSum[w] : 0;
+      carry += warpSum[w];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int i = off + threadIdx.x * 4 + j;
+      if (i < tiles) b.tileBase[i] = run;
+      run += v[j];
     }
   }
-}
-
-// updatePrims (:398-436): side of every prim of a split node
-template <int D>
-__global__ void side_kernel(BuildBufs b, int64_t n, uint32_t pb, uint32_t pe, int cur)
-{
-  const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (p >= n) return;
-  const uint32_t node = b.nodeOf[cur][p];
-  uint32_t l = 0;
-  if (node >= pb && node < pe && b.isSplit[node - pb]) {
-    const int dim = b.sdim[node];
-    int side;
-    if (dim < 0)
-      side = int((uint32_t(p) - b.segBegin[node]) & 1u);
-    else
-      side = b.coord[cur][dim][p] >= b.spos[node];
-    l = side == 0;
+  if (threadIdx.x == 0) {
+    b.tileBase[tiles] = carry;
+    b.st->ticket = 0;
   }
-  b.fl[p] = l;
 }
 
+// The open nodes' split records and children: leaves, subtree roots, or open
+// nodes of the next level (empty boxes).
 template <int D>
-__global__ void move_kernel(BuildBufs b, int64_t n, uint32_t pb, uint32_t pe, int cur)
+__global__ void __launch_bounds__(128) children_kernel(BuildBufs b, int par, uint32_t level,
+                                                       uint32_t threshold)
 {
+  const uint32_t m = b.st->open[par];
+  const int nxt = par ^ 1;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+    const uint32_t begin = b.begin[par][i], count = b.count[par][i];
+    float pos;
+    const int dim = decide<D>(b.lo[par] + int64_t(i) * D, b.hi[par] + int64_t(i) * D, &pos);
+    const uint32_t pre = left_before(b, begin);
+    const uint32_t nl = left_before(b, begin + count) - pre;
+    const uint32_t boundary = begin + nl;
+    note_split(b, boundary, dim, pos, level, b.link[par][i]);
+    uint32_t code[2];
+    for (int s = 0; s < 2; s++) {
+      const uint32_t cb = s == 0 ? begin : boundary, cc = s == 0 ? nl : count - nl;
+      const uint32_t link = boundary * 2 + (s == 0);
+      code[s] = kDone;
+      if (cc <= threshold) {
+        note_leaf(b, cb, cc, level + 1, nxt, link);
+        atomicAdd(&b.st->leaves, 1u);
+        atomicMax(&b.st->maxLevel, level + 1);
+      } else if (cc <= kSub) {
+        b.roots[atomicAdd(&b.st->subRoots, 1u)] = SubRoot{cb, cc, level + 1, link, uint32_t(nxt)};
+      } else {
+        const uint32_t c = atomicAdd(&b.st->open[nxt], 1u);
+        code[s] = c;
+        b.begin[nxt][c] = cb;
+        b.count[nxt][c] = cc;
+        b.link[nxt][c] = link;
+        for (int d = 0; d < D; d++) {
+          b.lo[nxt][int64_t(c) * D + d] = enc(+FLT_MAX);
+          b.hi[nxt][int64_t(c) * D + d] = enc(-FLT_MAX);
+        }
+      }
+    }
+    b.move[i] = make_uint4(begin, pre, nl, 0u);
+    b.codes[i] = make_uint2(code[0], code[1]);
+  }
+}
+
+// Every prim of an open node to its place in its child's segment; boxes of
+// the children that stay open.
+template <int D>
+__global__ void __launch_bounds__(256) move_kernel(BuildBufs b, int64_t n, int par)
+{
+  if (b.st->open[par] == 0) return;
   const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  const bool valid = p < n;
-  bool moving = false;
-  uint32_t child = 0;
+  const int nxt = par ^ 1;
+  uint32_t code = kDone;
   float pt[D];
 #pragma unroll
   for (int d = 0; d < D; d++) pt[d] = 0.f;
-  if (valid) {
-    const uint32_t node = b.nodeOf[cur][p];
-    const uint32_t prim = b.prim[cur][p];
-    int64_t dst = p;
-    uint32_t nodeOut = node;
-    if (node >= pb && node < pe && b.isSplit[node - pb]) {
-      const uint32_t sb = b.segBegin[node];
-      const uint32_t cnt = b.count[node];
-      const uint32_t nl = b.fl[sb + cnt] - b.fl[sb];
-      const uint32_t first = b.out[node].offset;
-      const bool isL = (b.fl[p + 1] - b.fl[p]) != 0;
-      // every prim of a split node goes left or right: its right-side rank
-      // is its rank in the segment minus its left-side rank
-      const uint32_t lBefore = b.fl[p] - b.fl[sb];
-      if (isL) {
-        dst = sb + lBefore;
-        nodeOut = first;
-      } else {
-        dst = sb + nl + (uint32_t(p) - sb - lBefore);
-        nodeOut = first + 1;
-      }
-      moving = true;
-      child = nodeOut;
+  if (p < n) {
+    const uint32_t node = b.nodeOf[par][p];
+    if (node == kDone) {
+      b.nodeOf[nxt][p] = kDone;
+    } else {
+      const uint4 mv = b.move[node];
+      const uint2 cd = b.codes[node];
+      const uint32_t before = left_before(b, uint32_t(p)) - mv.y;
+      const bool isL = (b.bits[p >> 5] >> (p & 31)) & 1u;
+      // a prim of a split node goes left or right: its right-side rank is its
+      // rank in the segment minus its left-side rank
+      const uint32_t dst = isL ? mv.x + before : mv.x + mv.z + (uint32_t(p) - mv.x - before);
+      code = isL ? cd.x : cd.y;
+      b.prim[nxt][dst] = b.prim[par][p];
+      b.nodeOf[nxt][dst] = code;
 #pragma unroll
       for (int d = 0; d < D; d++) {
-        pt[d] = b.coord[cur][d][p];
-        b.coord[cur ^ 1][d][dst] = pt[d];  // leaves' prims need no coordinates
+        pt[d] = b.coord[par][d][p];
+        b.coord[nxt][d][dst] = pt[d];
       }
     }
-    b.prim[cur ^ 1][dst] = prim;
-    b.nodeOf[cur ^ 1][dst] = nodeOut;
   }
-  block_grow<D>(b.lo, b.hi, child, moving, pt);
+  block_grow<D>(b.lo[nxt], b.hi[nxt], code, code != kDone, pt);
 }
 
-__global__ void child_counts_kernel(BuildBufs b, uint32_t pb, uint32_t pe)
-{
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= pe - pb || !b.isSplit[t]) return;
-  const uint32_t node = pb + t;
-  const uint32_t sb = b.segBegin[node], cnt = b.count[node];
-  const uint32_t nl = b.fl[sb + cnt] - b.fl[sb];
-  const uint32_t first = b.out[node].offset;
-  b.count[first] = nl;
-  b.count[first + 1] = cnt - nl;
-  b.segBegin[first] = sb;
-  b.segBegin[first + 1] = sb + nl;
-}
+// ---------------------------------------------------------------------------
+// one CTA finishes a subtree of at most kSub prims
+// ---------------------------------------------------------------------------
+constexpr int kSubThreads = 256;
+constexpr int kSubPer = kSub / kSubThreads;
+constexpr int kSubOpen = kSub / 2;  // open nodes hold at least two prims
 
-// leaf offsets in node-id order, then the prim list
-__global__ void leaf_counts_kernel(BuildBufs b, uint32_t numNodes, uint32_t *lc)
-{
-  const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
-  if (node >= numNodes) return;
-  lc[node] = (node != 1 && b.out[node].count > 0) ? b.out[node].count : 0u;
-}
-
-__global__ void leaf_offsets_kernel(BuildBufs b, uint32_t numNodes, const uint32_t *off)
-{
-  const uint32_t node = blockIdx.x * blockDim.x + threadIdx.x;
-  if (node >= numNodes || node == 1) return;
-  if (b.out[node].count > 0) b.out[node].offset = off[node];
-}
-
-__global__ void write_prims_kernel(BuildBufs b, int64_t n, int cur, const uint32_t *off,
-                                   uint32_t *primIDs)
-{
-  const int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (p >= n) return;
-  const uint32_t node = b.nodeOf[cur][p];
-  primIDs[off[node] + (uint32_t(p) - b.segBegin[node])] = b.prim[cur][p];
-}
+template <int D> struct SubtreeSmem {
+  float co[D][kSub];      // by input position
+  uint32_t pid[kSub];
+  int32_t lo[kSubOpen][D], hi[kSubOpen][D];
+  uint32_t link[2][kSubOpen];
+  uint16_t begin[2][kSubOpen], count[2][kSubOpen];
+  float pos[kSubOpen];
+  uint16_t pre[kSubOpen], nl[kSubOpen], code[kSubOpen][2];
+  int8_t dim[kSubOpen];
+  uint16_t ix[kSub], node[kSub];  // by position: input position, open node
+  uint32_t bits[kSub / 32], wordPre[kSub / 32 + 1];
+  uint32_t open[2], leaves, deepest;
+};
 
 template <int D>
-__global__ void bounds_out_kernel(BuildBufs b, float *bounds)
+__global__ void __launch_bounds__(kSubThreads) subtree_kernel(BuildBufs b, uint32_t threshold)
 {
-  if (threadIdx.x < D) {
-    bounds[threadIdx.x] = dec(b.lo[threadIdx.x]);
-    bounds[D + threadIdx.x] = dec(b.hi[threadIdx.x]);
+  extern __shared__ __align__(16) unsigned char raw[];
+  SubtreeSmem<D> &s = *reinterpret_cast<SubtreeSmem<D> *>(raw);
+  const SubRoot r = b.roots[blockIdx.x];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int n = int(r.count);
+  constexpr uint16_t kLeaf = 0xffff;
+  for (int p = tid; p < n; p += kSubThreads) {
+#pragma unroll
+    for (int d = 0; d < D; d++) s.co[d][p] = b.coord[r.parity][d][r.begin + p];
+    s.pid[p] = b.prim[r.parity][r.begin + p];
+    s.ix[p] = uint16_t(p);
+    s.node[p] = 0;
+  }
+  if (tid == 0) {
+    s.begin[0][0] = 0;
+    s.count[0][0] = uint16_t(n);
+    s.link[0][0] = r.link;
+    s.open[0] = 1;
+    s.leaves = 0;
+    s.deepest = r.level;
+  }
+  __syncthreads();
+  uint32_t level = r.level;
+  for (int par = 0;; par ^= 1, level++) {
+    const int m = int(s.open[par]);
+    if (m == 0) break;
+    for (int i = tid; i < m * D; i += kSubThreads) {
+      (&s.lo[0][0])[i] = enc(+FLT_MAX);
+      (&s.hi[0][0])[i] = enc(-FLT_MAX);
+    }
+    if (tid == 0) s.open[par ^ 1] = 0;
+    __syncthreads();
+    // positions p = (4 wid + j) * 32 + lane: a warp's are consecutive
+    uint16_t ix[kSubPer], nd[kSubPer];
+#pragma unroll
+    for (int j = 0; j < kSubPer; j++) {
+      const int p = (kSubPer * wid + j) * 32 + lane;
+      nd[j] = p < n ? s.node[p] : kLeaf;
+      ix[j] = p < n ? s.ix[p] : 0;
+      const uint32_t first = __shfl_sync(0xffffffffu, uint32_t(nd[j]), 0);
+      if (__all_sync(0xffffffffu, nd[j] == first)) {  // one node: reduced first
+        if (first != kLeaf) {
+#pragma unroll
+          for (int d = 0; d < D; d++) {
+            const int32_t e = enc(s.co[d][ix[j]]);
+            const int32_t l = __reduce_min_sync(0xffffffffu, e);
+            const int32_t h = __reduce_max_sync(0xffffffffu, e);
+            if (lane == 0) {
+              atomicMin(&s.lo[first][d], l);
+              atomicMax(&s.hi[first][d], h);
+            }
+          }
+        }
+      } else if (nd[j] != kLeaf) {
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+          const int32_t e = enc(s.co[d][ix[j]]);
+          atomicMin(&s.lo[nd[j]][d], e);
+          atomicMax(&s.hi[nd[j]][d], e);
+        }
+      }
+    }
+    __syncthreads();
+    for (int i = tid; i < m; i += kSubThreads) {
+      float pos;
+      s.dim[i] = int8_t(decide<D>(s.lo[i], s.hi[i], &pos));
+      s.pos[i] = pos;
+    }
+    __syncthreads();
+    bool left[kSubPer];
+#pragma unroll
+    for (int j = 0; j < kSubPer; j++) {
+      const int p = (kSubPer * wid + j) * 32 + lane;
+      left[j] = false;
+      if (nd[j] != kLeaf) {
+        const int dim = s.dim[nd[j]];
+        left[j] = dim < 0 ? ((p - s.begin[par][nd[j]]) & 1) == 0
+                          : !(s.co[dim][ix[j]] >= s.pos[nd[j]]);
+      }
+      const uint32_t w = __ballot_sync(0xffffffffu, left[j]);
+      if (lane == 0) s.bits[kSubPer * wid + j] = w;
+    }
+    __syncthreads();
+    if (wid == 0) {
+      const uint32_t c = __popc(s.bits[lane]);
+      uint32_t incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      s.wordPre[lane] = incl - c;
+      if (lane == 31) s.wordPre[32] = incl;
+    }
+    __syncthreads();
+    auto before = [&](int p) -> uint32_t {
+      return p == int(kSub) ? s.wordPre[32]
+                            : s.wordPre[p >> 5] + __popc(s.bits[p >> 5] & ((1u << (p & 31)) - 1u));
+    };
+    for (int i = tid; i < m; i += kSubThreads) {
+      const uint32_t begin = s.begin[par][i], count = s.count[par][i];
+      const uint32_t pre = before(int(begin)), nl = before(int(begin + count)) - pre;
+      const uint32_t boundary = r.begin + begin + nl;
+      note_split(b, boundary, s.dim[i], s.pos[i], level, s.link[par][i]);
+      s.pre[i] = uint16_t(pre);
+      s.nl[i] = uint16_t(nl);
+      for (int side = 0; side < 2; side++) {
+        const uint32_t cb = side == 0 ? begin : begin + nl, cc = side == 0 ? nl : count - nl;
+        const uint32_t link = boundary * 2 + (side == 0);
+        if (cc <= threshold) {
+          note_leaf(b, r.begin + cb, cc, level + 1, r.parity, link);
+          s.code[i][side] = kLeaf;
+          atomicAdd(&s.leaves, 1u);
+          s.deepest = level + 1;
+        } else {
+          const uint32_t c = atomicAdd(&s.open[par ^ 1], 1u);
+          s.begin[par ^ 1][c] = uint16_t(cb);
+          s.count[par ^ 1][c] = uint16_t(cc);
+          s.link[par ^ 1][c] = link;
+          s.code[i][side] = uint16_t(c);
+        }
+      }
+    }
+    __syncthreads();
+    // every thread holds its positions' prims in registers: moved in place
+#pragma unroll
+    for (int j = 0; j < kSubPer; j++) {
+      const int p = (kSubPer * wid + j) * 32 + lane;
+      if (nd[j] == kLeaf) continue;
+      const int i = nd[j];
+      const int begin = s.begin[par][i];
+      const int bf = int(before(p)) - int(s.pre[i]);
+      const int dst = left[j] ? begin + bf : begin + int(s.nl[i]) + (p - begin - bf);
+      s.ix[dst] = ix[j];
+      s.node[dst] = s.code[i][left[j] ? 0 : 1];
+    }
+    __syncthreads();
+  }
+  for (int p = tid; p < n; p += kSubThreads)
+    b.prim[r.parity][r.begin + p] = s.pid[s.ix[p]];
+  if (tid == 0) {
+    atomicAdd(&b.st->leaves, s.leaves);
+    atomicMax(&b.st->maxLevel, s.deepest);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// numbering
+// ---------------------------------------------------------------------------
+__global__ void iota_kernel(uint32_t *v, int64_t n)
+{
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x)
+    v[i] = uint32_t(i);
+}
+
+// node 1 is the reference's empty dummy (initState, :276-290)
+__device__ inline uint32_t node_id(uint32_t rank) { return rank == 0 ? 0u : rank + 1u; }
+
+// each place's node number, and the prims of the leaves by node number
+__global__ void number_kernel(BuildBufs b, const uint32_t *__restrict__ place, uint32_t nodes,
+                              uint32_t *id, uint32_t *leafPrims)
+{
+  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= nodes) return;
+  const uint32_t p = place[r];
+  id[p] = node_id(r);
+  leafPrims[node_id(r)] = (p & 1) ? 0u : b.leaf[p >> 1] & 0x7fffffffu;
+  if (r == 0) leafPrims[1] = 0;
+}
+
+// node records and the leaves' prim lists (a leaf of more than 16 prims by
+// its whole warp)
+__global__ void __launch_bounds__(256) write_kernel(BuildBufs b,
+                                                    const uint32_t *__restrict__ place,
+                                                    uint32_t nodes,
+                                                    const uint32_t *__restrict__ id,
+                                                    const uint32_t *__restrict__ offset,
+                                                    Node *out, uint32_t *primIDs)
+{
+  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t count = 0, first = 0, to = 0, parity = 0;
+  if (r < nodes) {
+    const uint32_t p = place[r];
+    Node o;
+    if (p & 1) {
+      const uint32_t boundary = (p + 1) >> 1;
+      o.pos = b.splitPos[boundary];
+      o.offset = id[b.splitChild[boundary]];
+      o.count = 0;
+      o.dim = int16_t(b.splitDim[boundary]);
+    } else {
+      first = p >> 1;
+      count = b.leaf[first] & 0x7fffffffu;
+      parity = b.leaf[first] >> 31;
+      to = offset[node_id(r)];
+      o.pos = 0.f;
+      o.offset = to;
+      o.count = uint16_t(count);
+      o.dim = 0;
+    }
+    out[node_id(r)] = o;
+    if (r == 0) out[1] = Node{0.f, 0u, 0, 0};
+  }
+  if (count <= 16)
+    for (uint32_t j = 0; j < count; j++) primIDs[to + j] = b.prim[parity][first + j];
+  for (unsigned big = __ballot_sync(0xffffffffu, count > 16); big; big &= big - 1) {
+    const int l = __ffs(big) - 1;
+    const uint32_t c = __shfl_sync(0xffffffffu, count, l);
+    const uint32_t f = __shfl_sync(0xffffffffu, first, l);
+    const uint32_t t = __shfl_sync(0xffffffffu, to, l);
+    const uint32_t *src = b.prim[__shfl_sync(0xffffffffu, parity, l)];
+    for (uint32_t j = threadIdx.x & 31; j < c; j += 32) primIDs[t + j] = src[f + j];
   }
 }
 
@@ -395,105 +732,129 @@ int build_impl(const void *pts, int64_t n, const Layout &L, int threshold,
   if (threshold == 0) threshold = 8;  // spatial-kdtree.h:505-506
   if (threshold < 1 || threshold > 65535) return CUKD_ERR_INVALID_ARGUMENT;
   TempArena arena(st, mem);
-  const int64_t cap = 2 * n + 2;
   BuildBufs b = {};
   b.data = (const uint8_t *)pts;
   b.stride = L.stride;
   b.poff = L.poff;
-  CKB_TRY(arena.alloc(&b.count, cap));
-  CKB_TRY(arena.alloc(&b.segBegin, cap));
-  CKB_TRY(arena.alloc(&b.lo, cap * D));
-  CKB_TRY(arena.alloc(&b.hi, cap * D));
-  CKB_TRY(arena.alloc(&b.sdim, cap));
-  CKB_TRY(arena.alloc(&b.spos, cap));
-  CKB_TRY(arena.alloc(&b.isSplit, cap));
-  CKB_TRY(arena.alloc(&b.splitRank, cap));
+  // open nodes hold more than kSub prims each
+  const int64_t cap = std::max<int64_t>(1, n / kSub + 1);
+  const int tiles = int(std::max<int64_t>(1, div_up(n, kSideTile)));
+  const int64_t np = std::max<int64_t>(n, 1);
+  uint32_t *key2 = nullptr, *place = nullptr, *place2 = nullptr;
+  CKB_TRY(arena.alloc(&b.st, 1));
   for (int x = 0; x < 2; x++) {
-    CKB_TRY(arena.alloc(&b.prim[x], n));
-    CKB_TRY(arena.alloc(&b.nodeOf[x], n));
-    for (int d = 0; d < D; d++) CKB_TRY(arena.alloc(&b.coord[x][d], n));
+    CKB_TRY(arena.alloc(&b.begin[x], cap));
+    CKB_TRY(arena.alloc(&b.count[x], cap));
+    CKB_TRY(arena.alloc(&b.link[x], cap));
+    CKB_TRY(arena.alloc(&b.lo[x], cap * D));
+    CKB_TRY(arena.alloc(&b.hi[x], cap * D));
+    CKB_TRY(arena.alloc(&b.prim[x], np));
+    CKB_TRY(arena.alloc(&b.nodeOf[x], np));
+    for (int d = 0; d < D; d++) CKB_TRY(arena.alloc(&b.coord[x][d], np));
   }
-  CKB_TRY(arena.alloc(&b.fl, n + 1));
-  CKB_TRY(arena.alloc(&b.total, 4));
-  Node *nodesFull = nullptr;
-  CKB_TRY(arena.alloc(&nodesFull, cap));
-  b.out = nodesFull;
-  // the per-pass split count is read into pageable memory (a 4-byte copy
-  // followed by a stream sync anyway; a pinned allocation per build cost more)
-  uint32_t hostTotalVal = 0;
-  uint32_t *hostTotal = &hostTotalVal;
-
+  CKB_TRY(arena.alloc(&b.move, cap));
+  CKB_TRY(arena.alloc(&b.codes, cap));
+  CKB_TRY(arena.alloc(&b.bits, int64_t(tiles) * (kSideTile / 32)));
+  CKB_TRY(arena.alloc(&b.wordPre, int64_t(tiles) * (kSideTile / 32)));
+  CKB_TRY(arena.alloc(&b.tileBase, tiles + 1));
+  CKB_TRY(arena.alloc(&b.roots, np / 2 + 1));  // at least two prims each
+  CKB_TRY(arena.alloc(&b.key, 2 * np));
+  CKB_TRY(arena.alloc(&key2, 2 * np));
+  CKB_TRY(arena.alloc(&place, 2 * np));
+  CKB_TRY(arena.alloc(&place2, 2 * np));
+  CKB_TRY(arena.alloc(&b.splitChild, np));
+  CKB_TRY(arena.alloc(&b.splitPos, np));
+  CKB_TRY(arena.alloc(&b.splitDim, np));
+  CKB_TRY(arena.alloc(&b.leaf, np));
   // root: empty box, then grown by every prim (initPrims, :300-314)
   {
-    std::vector<int32_t> lo(D, enc(+FLT_MAX)), hi(D, enc(-FLT_MAX));
-    CKB_CUDA(cudaMemcpyAsync(b.lo, lo.data(), sizeof(int32_t) * D, cudaMemcpyHostToDevice, st));
-    CKB_CUDA(cudaMemcpyAsync(b.hi, hi.data(), sizeof(int32_t) * D, cudaMemcpyHostToDevice, st));
+    int32_t box[2 * D];
+    for (int d = 0; d < D; d++) {
+      box[d] = enc(+FLT_MAX);
+      box[D + d] = enc(-FLT_MAX);
+    }
+    CKB_CUDA(cudaMemcpyAsync(b.lo[0], box, sizeof(int32_t) * D, cudaMemcpyHostToDevice, st));
+    CKB_CUDA(cudaMemcpyAsync(b.hi[0], box + D, sizeof(int32_t) * D, cudaMemcpyHostToDevice, st));
   }
-  const unsigned nb = unsigned(std::max<int64_t>(1, div_up(n, 256)));
+  // places without a node sort behind every level
+  CKB_CUDA(cudaMemsetAsync(b.key, 0xff, sizeof(uint32_t) * 2 * np, st));
+  const unsigned nb = unsigned(div_up(np, 256));
   init_kernel<D><<<nb, 256, 0, st>>>(b, n);
   CKB_CHECK_LAUNCH();
-  root_setup_kernel<D><<<1, 32, 0, st>>>(b, n);
+  // the root's box is the tree's: kept before its buffer is used again
+  int32_t *box = nullptr;
+  CKB_TRY(arena.alloc(&box, 2 * D));
+  CKB_CUDA(cudaMemcpyAsync(box, b.lo[0], sizeof(int32_t) * D, cudaMemcpyDeviceToDevice, st));
+  CKB_CUDA(cudaMemcpyAsync(box + D, b.hi[0], sizeof(int32_t) * D, cudaMemcpyDeviceToDevice, st));
+  root_kernel<<<1, 1, 0, st>>>(b, uint32_t(n), uint32_t(threshold));
   CKB_CHECK_LAUNCH();
 
-  uint32_t pb = 0, pe = 1, numNodes = 2;  // open nodes this pass: [pb, pe)
-  int cur = 0;
-  bool first = true;
-  while (pe > pb) {
-    const uint32_t m = pe - pb;
-    const unsigned mb = unsigned(div_up(m, 256));
-    decide_kernel<D><<<mb, 256, 0, st>>>(b, pb, pe, threshold);
-    CKB_CHECK_LAUNCH();
-    CKB_TRY(exclusive_scan_u32(b.isSplit, b.splitRank, m, b.total, st, &arena));
-    CKB_CUDA(cudaMemcpyAsync(hostTotal, b.total, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    CKB_CUDA(cudaStreamSynchronize(st));
-    const uint32_t numSplit = *hostTotal;
-    if (numSplit == 0) break;
-    // node 1 is the reference's dummy, so the root's children start at 2
-    const uint32_t childBase = first ? 2u : pe;
-    children_kernel<D><<<mb, 256, 0, st>>>(b, pb, pe, childBase);
-    CKB_CHECK_LAUNCH();
-    side_kernel<D><<<nb, 256, 0, st>>>(b, n, pb, pe, cur);
-    CKB_CHECK_LAUNCH();
-    CKB_TRY(exclusive_scan_u32(b.fl, b.fl, n + 1, nullptr, st, &arena));
-    child_counts_kernel<<<mb, 256, 0, st>>>(b, pb, pe);
-    CKB_CHECK_LAUNCH();
-    move_kernel<D><<<nb, 256, 0, st>>>(b, n, pb, pe, cur);
-    CKB_CHECK_LAUNCH();
-    cur ^= 1;
-    numNodes = childBase + 2 * numSplit;
-    pb = childBase;
-    pe = numNodes;
-    first = false;
+  // ---- the level phase: the levels a balanced tree would need, two more,
+  // then four at a time until no open node is left (a launch without open
+  // nodes returns at once)
+  uint32_t subRoots = n <= threshold ? 0 : 1;
+  const int64_t big = std::max<int64_t>(kSub, threshold);
+  if (n > big) {
+    int batch = 2;
+    for (int64_t c = n; c > big; c = div_up(c, 2)) batch++;
+    BuildState hs = {};
+    uint32_t level = 0;
+    do {
+      for (int i = 0; i < batch; i++, level++) {
+        const int par = int(level & 1);
+        side_kernel<D><<<unsigned(tiles), 256, 0, st>>>(b, n, par, tiles);
+        CKB_CHECK_LAUNCH();
+        const int64_t open = level < 40 ? std::min<int64_t>(cap, int64_t(1) << level) : cap;
+        children_kernel<D><<<unsigned(std::min<int64_t>(div_up(open, 128), kNumSMs * 8)), 128, 0,
+                             st>>>(b, par, level, uint32_t(threshold));
+        CKB_CHECK_LAUNCH();
+        move_kernel<D><<<nb, 256, 0, st>>>(b, n, par);
+        CKB_CHECK_LAUNCH();
+      }
+      CKB_CUDA(cudaMemcpyAsync(&hs, b.st, sizeof(hs), cudaMemcpyDeviceToHost, st));
+      CKB_CUDA(cudaStreamSynchronize(st));
+      batch = 4;
+    } while (hs.open[level & 1] != 0);
+    subRoots = hs.subRoots;
   }
-
-  // leaf prim lists in node-id order
-  uint32_t *lc = nullptr;
-  CKB_TRY(arena.alloc(&lc, numNodes + 1));
-  const unsigned tb = unsigned(div_up(numNodes, 256));
-  leaf_counts_kernel<<<tb, 256, 0, st>>>(b, numNodes, lc);
+  // ---- subtrees
+  if (subRoots > 0) {
+    constexpr int smem = int(sizeof(SubtreeSmem<D>));
+    CKB_CUDA(cudaFuncSetAttribute(subtree_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  smem));
+    subtree_kernel<D><<<subRoots, kSubThreads, smem, st>>>(b, uint32_t(threshold));
+    CKB_CHECK_LAUNCH();
+  }
+  // ---- numbering: nodes by level, then from left to right
+  iota_kernel<<<unsigned(std::min<int64_t>(div_up(2 * np, 256), kNumSMs * 16)), 256, 0, st>>>(
+      place, 2 * np);
   CKB_CHECK_LAUNCH();
-  CKB_TRY(exclusive_scan_u32(lc, lc, numNodes, nullptr, st, &arena));
-  leaf_offsets_kernel<<<tb, 256, 0, st>>>(b, numNodes, lc);
+  BuildState hs = {};
+  int32_t hb[2 * D];
+  CKB_CUDA(cudaMemcpyAsync(&hs, b.st, sizeof(hs), cudaMemcpyDeviceToHost, st));
+  CKB_CUDA(cudaMemcpyAsync(hb, box, sizeof(hb), cudaMemcpyDeviceToHost, st));
+  CKB_CUDA(cudaStreamSynchronize(st));
+  // (a box halves an extent per level: a depth of a few thousand at most)
+  CKB_TRY(radix_sort_pairs(b.key, place, key2, place2, 2 * np, hs.maxLevel < 255 ? 8 : 16, st,
+                           &arena));
+  const uint32_t count = n > 0 ? 2 * hs.leaves - 1 : 1;
+  const uint32_t numNodes = count + 1;
+  uint32_t *id = key2, *off = nullptr;
+  CKB_TRY(arena.alloc(&off, numNodes + 1));
+  const unsigned tb = unsigned(div_up(count, 256));
+  number_kernel<<<tb, 256, 0, st>>>(b, place, count, id, off);
   CKB_CHECK_LAUNCH();
+  CKB_TRY(exclusive_scan_u32(off, off, numNodes, nullptr, st, &arena));
 
   void *nodes = nullptr, *prims = nullptr;
   CKB_TRY(alloc_out(mem, st, &nodes, sizeof(Node) * numNodes));
-  const int rcP = alloc_out(mem, st, &prims, sizeof(uint32_t) * std::max<int64_t>(n, 1));
+  const int rcP = alloc_out(mem, st, &prims, sizeof(uint32_t) * np);
   if (rcP != CUKD_OK) {
     if (mem && mem->release) mem->release(mem->ctx, nodes, st); else cudaFreeAsync(nodes, st);
     return rcP;
   }
-  write_prims_kernel<<<nb, 256, 0, st>>>(b, n, cur, lc, (uint32_t *)prims);
+  write_kernel<<<tb, 256, 0, st>>>(b, place, count, id, off, (Node *)nodes, (uint32_t *)prims);
   CKB_CHECK_LAUNCH();
-  CKB_CUDA(cudaMemcpyAsync(nodes, nodesFull, sizeof(Node) * numNodes, cudaMemcpyDeviceToDevice,
-                           st));
-  float *bnd = nullptr;
-  CKB_TRY(arena.alloc(&bnd, 2 * D));
-  bounds_out_kernel<D><<<1, 32, 0, st>>>(b, bnd);
-  CKB_CHECK_LAUNCH();
-  float hb[8];
-  CKB_CUDA(cudaMemcpyAsync(hb, bnd, sizeof(float) * 2 * D, cudaMemcpyDeviceToHost, st));
-  CKB_CUDA(cudaStreamSynchronize(st));
   tree->nodes = (Node *)nodes;
   tree->prim_ids = (uint32_t *)prims;
   tree->data = pts;
@@ -502,8 +863,8 @@ int build_impl(const void *pts, int64_t n, const Layout &L, int threshold,
   tree->num_dims = D;
   for (int i = 0; i < 8; i++) tree->bounds[i] = 0.f;
   for (int d = 0; d < D; d++) {
-    tree->bounds[d] = hb[d];
-    tree->bounds[4 + d] = hb[D + d];
+    tree->bounds[d] = dec(hb[d]);
+    tree->bounds[4 + d] = dec(hb[D + d]);
   }
   return CUKD_OK;
 }
