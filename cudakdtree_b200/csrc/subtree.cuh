@@ -273,6 +273,192 @@ __device__ void sub_radix_sort_all(SubSmem<D, TILE, NT> &S, int m)
   }
 }
 
+// left-side size of a left-balanced tree of sz >= 1 nodes
+__device__ __forceinline__ int left_of(int sz)
+{
+  if (sz == 1) return 0;
+  const int h = 32 - __clz(sz), half = 1 << (h - 2);
+  return half - 1 + min(sz - ((1 << (h - 1)) - 1), half);
+}
+
+// The bottom levels: one warp finishes the subtree under node g (level lvl,
+// local index u, at most 32 points at positions bt.. of the lists), a point
+// per lane.  A point's rank along a dimension is its place in that
+// dimension's sorted list; a segment's members are a bit mask over those
+// ranks, one mask per dimension, so a level is a popc for the rank in the
+// segment and, per dimension, a shuffle and two ballots that split the mask
+// -- no barriers and no lists to partition.  (Against carrying the CTA-wide
+// levels down to single points: PLACEHOLDER)
+template <int SC, int D, int TILE, int NT, class Src>
+__device__ __forceinline__ void warp_levels(Src &src, int64_t n, int64_t g, int lvl, int u, int bt,
+                                            int cur, bool explicitDims, SubSmem<D, TILE, NT> &S)
+{
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  int sz = int(subtree_size(g, n));
+  bool act = lane < sz;
+  const int e = act ? S.list[cur][0][bt + lane] : 0;
+  uint32_t key[D];
+#pragma unroll
+  for (int d = 0; d < D; d++) key[d] = S.key[d][e];
+  const uint32_t idx = S.idx[e];
+  int rank[D], at[D];  // this point's rank, and the lane of the point of rank `lane`
+  rank[0] = at[0] = lane;
+#pragma unroll
+  for (int d = 1; d < D; d++) {
+    const int ed = act ? S.list[cur][d][bt + lane] : 0;
+    if (act) S.flag[e] = uint8_t(lane);
+    __syncwarp();
+    at[d] = act ? int(S.flag[ed]) : lane;
+    __syncwarp();
+    if (act) S.flag[ed] = uint8_t(lane);
+    __syncwarp();
+    rank[d] = act ? int(S.flag[e]) : lane;
+    __syncwarp();
+  }
+  // the ancestors' dims, nearest first, each once (the words of the
+  // composite key behind the own dim's); explicit dims: the domain box
+  uint32_t recent = 0;
+  int nrecent = 0;
+  {
+    int c = u;
+    int64_t ga = g;
+    while (ga > 0 && nrecent < D) {
+      int da;
+      if (c > 0) {
+        c = (c - 1) >> 1;
+        da = S.locDim[c];
+      } else {
+        da = explicitDims ? src.anc_dim((ga - 1) >> 1) : rr_dim((ga - 1) >> 1, D);
+      }
+      ga = (ga - 1) >> 1;
+      bool seen = false;
+      for (int i = 0; i < nrecent; i++) seen |= int((recent >> (4 * i)) & 15u) == da;
+      if (!seen) recent |= uint32_t(da) << (4 * nrecent++);
+    }
+  }
+  uint32_t lo[D], hi[D];
+  if (explicitDims) {
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+      lo[d] = S.rootLo[d];
+      hi[d] = S.rootHi[d];
+    }
+    for (int c = u; c > 0; c = (c - 1) >> 1) {
+      const int p = (c - 1) >> 1, pd = S.locDim[p];
+      const uint32_t pc = S.key[pd][S.locPivot[p]];
+#pragma unroll
+      for (int d = 0; d < D; d++)
+        if (d == pd) {
+          if (c & 1)
+            hi[d] = min(hi[d], pc);
+          else
+            lo[d] = max(lo[d], pc);
+        }
+    }
+  }
+  const uint32_t all = sz >= 32 ? FULL : (1u << sz) - 1u;
+  uint32_t members = all;  // of this lane's segment, as lanes
+  uint32_t seg[D];         // as ranks, per dimension
+#pragma unroll
+  for (int d = 0; d < D; d++) seg[d] = all;
+  for (int left_levels = 32 - __clz(sz); left_levels > 0; left_levels--) {
+    const int r = act ? left_of(sz) : 0;
+    const int dim = explicitDims ? Scalar<SC>::widest(lo, hi, D) : lvl % D;
+    uint32_t kd = key[0], sd = seg[0];
+    int rk = rank[0];
+#pragma unroll
+    for (int d = 1; d < D; d++)
+      if (d == dim) {
+        kd = key[d];
+        sd = seg[d];
+        rk = rank[d];
+      }
+    int pos = __popc(sd & ((1u << rk) - 1u));  // rank in the segment
+    bool pivot = act && pos == r;
+    int pl = __ffs(__ballot_sync(FULL, pivot) & members) - 1;
+    const uint32_t pk = __shfl_sync(FULL, kd, act ? pl : lane);
+    const bool run = act && kd == pk;
+    if (__any_sync(FULL, run && !pivot)) {
+      // equal coordinates around a pivot: its run is ranked by the
+      // composite key
+      uint32_t word[D];
+      int words = 0;
+#pragma unroll
+      for (int w = 0; w < D; w++) {
+        word[w] = 0;
+        const int dw = int((recent >> (4 * w)) & 15u);
+        if (w < nrecent && dw != dim) {
+          uint32_t v = key[0];
+#pragma unroll
+          for (int d = 1; d < D; d++) v = d == dw ? key[d] : v;
+          word[w] = v;
+        }
+        words = w < nrecent ? w + 1 : words;
+      }
+      const uint32_t runs = __ballot_sync(FULL, run);
+      const int below = __popc(__ballot_sync(FULL, act && kd < pk) & members);
+      int before = 0;
+      for (int o = 0; o < 32; o++) {
+        bool less = false, decided = false;
+#pragma unroll
+        for (int w = 0; w < D; w++) {
+          const uint32_t ow = __shfl_sync(FULL, word[w], o);
+          if (w < words && !decided && ow != word[w]) {
+            less = ow < word[w];
+            decided = true;
+          }
+        }
+        const uint32_t oi = __shfl_sync(FULL, idx, o);
+        if (!decided) less = oi < idx;
+        before += int(less && ((runs & members) >> o & 1u));
+      }
+      if (run) pos = below + before;
+      pivot = act && pos == r;
+    }
+    const bool left = act && pos < r, right = act && pos > r;
+    if (pivot) {
+      S.locDim[u] = uint8_t(dim);
+      src.settle(g, u, e, dim, S);
+    }
+    const int side = left ? 1 : (right ? 2 : 0);
+    const uint32_t lefts = __ballot_sync(FULL, left), rights = __ballot_sync(FULL, right);
+    members &= left ? lefts : rights;
+    act = left || right;
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+      const int so = __shfl_sync(FULL, side, at[d]);
+      const uint32_t l = __ballot_sync(FULL, so == 1), rr = __ballot_sync(FULL, so == 2);
+      seg[d] &= left ? l : rr;
+    }
+    if (explicitDims) {
+#pragma unroll
+      for (int d = 0; d < D; d++)
+        if (d == dim) {
+          if (left)
+            hi[d] = min(hi[d], pk);
+          else
+            lo[d] = max(lo[d], pk);
+        }
+    }
+    // dim to the front of the recent ones
+    {
+      uint32_t kept = uint32_t(dim);
+      int k = 1;
+      for (int i = 0; i < nrecent; i++) {
+        const uint32_t x = (recent >> (4 * i)) & 15u;
+        if (int(x) != dim) kept |= x << (4 * k++);
+      }
+      recent = kept;
+      nrecent = k;
+    }
+    sz = left ? r : sz - 1 - r;
+    g = 2 * g + (left ? 1 : 2);
+    u = 2 * u + (left ? 1 : 2);
+    lvl++;
+  }
+}
+
 // Finishes the subtree under node s (level L0) of a tree of n records.
 // Src supplies the data and takes the result:
 //   src.load(S, m)             fills S.key[d][i] and S.idx[i] (the composite
@@ -309,6 +495,12 @@ __device__ void subtree_body(Src &src, int64_t n, int L0, int64_t s, bool explic
     const int64_t base0 = seg_begin(g0, lvl, n);
     const int nsub = 1 << j;
     int nexist = int(min(int64_t(nsub), max(int64_t(0), n - g0)));
+    if (subtree_size(g0, n) <= 32) {  // the level's largest
+      for (int t = wid; t < nexist; t += NT / 32)
+        warp_levels<SC, D, TILE, NT>(src, n, g0 + t, lvl, (1 << j) - 1 + t,
+                                     int(seg_begin(g0 + t, lvl, n) - base0), cur, explicitDims, S);
+      break;
+    }
     uint32_t &qcount = S.qcount[j & 1];
     if (tid == 0) S.qcount[(j + 1) & 1] = 0;  // the next level's; read last a level ago
     // A: per subtree, its dim, pivot rank position and equal-key run
