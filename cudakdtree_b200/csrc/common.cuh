@@ -5,6 +5,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "cukd_b200.h"
@@ -61,19 +62,37 @@ struct TempArena {
   const cukd_mem_resource *mem;
   cudaMemPool_t pool;  // without a caller's resource: this pool, else the device's default
   std::vector<void *> ptrs;
+  uint8_t *block = nullptr;  // what is left of a reserved block
+  size_t left = 0;
   TempArena(cudaStream_t s, const cukd_mem_resource *m, cudaMemPool_t p = nullptr)
       : stream(s), mem(m), pool(p)
   {
     if (!mem || !mem->alloc) keep_default_pool_memory();
   }
   ~TempArena() { release_all(); }
+  static size_t rounded(size_t bytes) { return (std::max<size_t>(bytes, 16) + 255) & ~size_t(255); }
+  // One block for the allocations that follow (what does not fit it is
+  // allocated by itself): twenty stream-ordered allocations of a build cost
+  // the host as much as its launches.
+  int reserve(size_t bytes)
+  {
+    uint8_t *p = nullptr;
+    CKB_TRY(alloc(&p, bytes));
+    block = p;
+    left = bytes;
+    return CUKD_OK;
+  }
   template <typename T>
   int alloc(T **out, size_t count)
   {
     void *p = nullptr;
-    size_t bytes = count * sizeof(T);
-    if (bytes == 0) bytes = 16;
-    bytes = (bytes + 255) & ~size_t(255);
+    const size_t bytes = rounded(count * sizeof(T));
+    if (bytes <= left) {
+      *out = (T *)block;
+      block += bytes;
+      left -= bytes;
+      return CUKD_OK;
+    }
     void *use = nullptr;
     if (mem && mem->alloc) {
       // the builder's bulk copies need 16-byte-aligned arrays, and a caller's
@@ -103,6 +122,7 @@ struct TempArena {
         cudaFreeAsync(p, stream);
     }
     ptrs.clear();
+    left = 0;
   }
 };
 

@@ -48,6 +48,9 @@
 struct cukd_radius_model_s;
 
 namespace ckb {
+int query_order(const void *queries, int64_t n, int scalar, int D, const void *d_bounds,
+                const float *lo, const float *hi, const int32_t **order, cudaStream_t st,
+                TempArena *arena);
 namespace learned {
 
 constexpr int S = 32;             // samples per CTA in training
@@ -718,11 +721,13 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   a.out_d2 = d_out_d2;
   a.visits = d_visits;
   a.block_size = p->block_size;
-  if ((p->flags & CUKD_QUERY_MORTON) && nq > 1 && L.scalar == CUKD_FLOAT32) {
+  if ((p->flags & CUKD_QUERY_MORTON) && nq > 1 && d_world_bounds) {
+    CKB_TRY(query_order(d_queries, nq, L.scalar, L.D, d_world_bounds, nullptr, nullptr, &a.order,
+                        st, &arena));
+  } else if ((p->flags & CUKD_QUERY_MORTON) && nq > 1 && L.scalar == CUKD_FLOAT32) {
     int32_t *perm = nullptr;
     CKB_TRY(arena.alloc(&perm, nq));
-    CKB_TRY(cukd_morton_order((const float *)d_queries, nq, L.D, (const float *)d_world_bounds,
-                              perm, st, mem));
+    CKB_TRY(cukd_morton_order((const float *)d_queries, nq, L.D, nullptr, perm, st, mem));
     a.order = perm;
   }
   int *ctr = nullptr;

@@ -187,6 +187,9 @@ int run_query(const QArgs &a, int scalar, int D, int method, int kind, cudaStrea
 
 int morton_order_impl(const float *pts, int64_t n, int D, const float *bounds, int32_t *perm,
                       cudaStream_t st, const cukd_mem_resource *mem);
+int query_order(const void *queries, int64_t n, int scalar, int D, const void *d_bounds,
+                const float *lo, const float *hi, const int32_t **order, cudaStream_t st,
+                TempArena *arena);
 
 
 static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout,
@@ -278,14 +281,14 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     CKB_TRY(run_tree_path(a, L.scalar, L.D, levels, codes, vals, st));
     CKB_TRY(radix_sort_pairs(codes, vals, codes2, vals2, nq, levels, st, &arena));
     a.order = (const int32_t *)vals;
+  } else if ((p->flags & CUKD_QUERY_MORTON) && nq > 1 && narrow && d_world_bounds) {
+    CKB_TRY(query_order(d_queries, nq, L.scalar, L.D, d_world_bounds, nullptr, nullptr, &a.order,
+                        st, &arena));
   } else if ((p->flags & CUKD_QUERY_MORTON) && nq > 1 && L.scalar == CUKD_FLOAT32 && narrow) {
+    // without the tree's bounds: over the queries' own (one more pass)
     int32_t *perm = nullptr;
     CKB_TRY(arena.alloc(&perm, nq));
-    // the Morton grid spans the tree's world bounds when the caller passes
-    // them (no bounds pass over the queries; queries outside are clamped to
-    // the box faces, which only coarsens their order), else the queries' own
-    CKB_TRY(morton_order_impl((const float *)d_queries, nq, L.D, (const float *)d_world_bounds,
-                              perm, st, mem));
+    CKB_TRY(morton_order_impl((const float *)d_queries, nq, L.D, nullptr, perm, st, mem));
     a.order = perm;
   }
   // fast exact path (see fast.cu): any visiting order, boundary-tie check,

@@ -11,6 +11,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kItems = 16;
 constexpr int kTileItems = kThreads * kItems;
+static_assert(kTileItems == kSortTile, "documented tile");
 
 __global__ void __launch_bounds__(kThreads) upsweep_kernel(const uint32_t *__restrict__ keys,
                                                            int64_t n, int shift, int numTiles,
@@ -85,6 +86,9 @@ __global__ void __launch_bounds__(kThreads) column_scan_kernel(uint32_t *counts,
 // digit's run from this tile are consecutive addresses.  (The earlier form
 // ranked 256 items at a time with three barriers each and wrote straight
 // to global memory: 180 us a pass over 10M keys in a cold ncu replay.)
+// IOTA: the values are the positions (vals is not read); KEYS: the sorted
+// keys are written, too.
+template <bool IOTA, bool KEYS>
 __global__ void __launch_bounds__(kThreads, 3) scatter_kernel(
     const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals, int64_t n, int shift,
     int numTiles, const uint32_t *__restrict__ offsets, const uint32_t *__restrict__ digitTotals,
@@ -106,13 +110,13 @@ __global__ void __launch_bounds__(kThreads, 3) scatter_kernel(
   // this warp's items in the tile: positions below lim are in the input
   const int64_t rem = n - wbase;
   const int lim = rem <= 0 ? 0 : (rem < kWarpItems ? int(rem) : kWarpItems);
-  const uint32_t *kw = keys + wbase, *vw = vals + wbase;
+  const uint32_t *kw = keys + wbase, *vw = IOTA ? nullptr : vals + wbase;
   uint32_t k[kItems], v[kItems];
 #pragma unroll
   for (int j = 0; j < kItems; j++) {
     const int i = j * 32 + lane;
     k[j] = i < lim ? kw[i] : 0u;
-    v[j] = i < lim ? vw[i] : 0u;
+    v[j] = IOTA ? uint32_t(wbase + i) : (i < lim ? vw[i] : 0u);
   }
   __syncthreads();
   const uint32_t ltMask = (1u << lane) - 1u;
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(kThreads, 3) scatter_kernel(
     const uint32_t key = sk[p];
     const uint32_t d = (key >> shift) & 255u;
     const uint32_t g = outBase[d] + uint32_t(p) - tileStart[d];
-    keysOut[g] = key;
+    if (KEYS) keysOut[g] = key;
     valsOut[g] = sv[p];
   }
 }
@@ -215,7 +219,7 @@ int radix_sort_pairs_ws(uint32_t *keys, uint32_t *vals, uint32_t *keys2, uint32_
     CKB_CHECK_LAUNCH();
     column_scan_kernel<<<256, kThreads, 0, st>>>(counts, numTiles, totals);
     CKB_CHECK_LAUNCH();
-    scatter_kernel<<<numTiles, kThreads, 0, st>>>(ka, va, n, shift, numTiles, counts, totals, kb,
+    scatter_kernel<false, true><<<numTiles, kThreads, 0, st>>>(ka, va, n, shift, numTiles, counts, totals, kb,
                                                   vb);
     CKB_CHECK_LAUNCH();
     std::swap(ka, kb);
@@ -224,6 +228,35 @@ int radix_sort_pairs_ws(uint32_t *keys, uint32_t *vals, uint32_t *keys2, uint32_
   if (ka != keys) {
     CKB_CUDA(cudaMemcpyAsync(keys, ka, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st));
     CKB_CUDA(cudaMemcpyAsync(vals, va, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st));
+  }
+  return CUKD_OK;
+}
+
+int radix_order(uint32_t *codes, uint32_t *codes2, uint32_t *vals, uint32_t *vals2, int64_t n,
+                int passes, uint32_t *counts, cudaStream_t st)
+{
+  const int numTiles = int(div_up(n, kTileItems));
+  uint32_t *totals = counts + int64_t(numTiles) * 256;
+  for (int pass = 0; pass < passes; pass++) {
+    const int shift = 8 * pass;
+    uint32_t *ka = pass & 1 ? codes2 : codes, *va = pass & 1 ? vals2 : vals;
+    uint32_t *kb = pass & 1 ? codes : codes2, *vb = pass & 1 ? vals : vals2;
+    if (pass > 0) {  // (the first digit's counts come with the codes)
+      upsweep_kernel<<<numTiles, kThreads, 0, st>>>(ka, n, shift, numTiles, counts);
+      CKB_CHECK_LAUNCH();
+    }
+    column_scan_kernel<<<256, kThreads, 0, st>>>(counts, numTiles, totals);
+    CKB_CHECK_LAUNCH();
+    if (pass == 0)
+      scatter_kernel<true, true><<<numTiles, kThreads, 0, st>>>(ka, va, n, shift, numTiles,
+                                                                counts, totals, kb, vb);
+    else if (pass < passes - 1)
+      scatter_kernel<false, true><<<numTiles, kThreads, 0, st>>>(ka, va, n, shift, numTiles,
+                                                                 counts, totals, kb, vb);
+    else
+      scatter_kernel<false, false><<<numTiles, kThreads, 0, st>>>(ka, va, n, shift, numTiles,
+                                                                  counts, totals, kb, vb);
+    CKB_CHECK_LAUNCH();
   }
   return CUKD_OK;
 }

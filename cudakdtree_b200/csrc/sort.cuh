@@ -16,4 +16,13 @@ int64_t radix_sort_counts(int64_t n);
 int radix_sort_pairs_ws(uint32_t *keys, uint32_t *vals, uint32_t *keys2, uint32_t *vals2,
                         int64_t n, int bits, uint32_t *counts, cudaStream_t st);
 
+// The stable order of n codes of 8 * passes bits (passes >= 2), left in vals2
+// after an odd number of passes, else in vals: the first digit's counts are
+// already in counts[digit * tiles + tile] (tiles of kSortTile codes), the last
+// pass leaves the keys out.  codes, codes2 and the other values are scratch;
+// counts has radix_sort_counts(n) entries.
+constexpr int kSortTile = 4096;
+int radix_order(uint32_t *codes, uint32_t *codes2, uint32_t *vals, uint32_t *vals2, int64_t n,
+                int passes, uint32_t *counts, cudaStream_t st);
+
 }  // namespace ckb

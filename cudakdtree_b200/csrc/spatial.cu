@@ -1035,8 +1035,9 @@ int query_impl(const SArgs &s, int method, int kind, cudaStream_t st)
 
 }  // namespace spatial
 
-int morton_order_impl(const float *pts, int64_t n, int D, const float *bounds, int32_t *perm,
-                      cudaStream_t st, const cukd_mem_resource *mem);
+int query_order(const void *queries, int64_t n, int scalar, int D, const void *d_bounds,
+                const float *lo, const float *hi, const int32_t **order, cudaStream_t st,
+                TempArena *arena);
 
 static int spatial_query(const cukd_spatial_tree *tree, const cukd_layout *layout,
                          const void *d_queries, int64_t nq, const cukd_query_params *p,
@@ -1079,10 +1080,8 @@ static int spatial_query(const cukd_spatial_tree *tree, const cukd_layout *layou
   }
   TempArena arena(st, mem);
   if ((p->flags & CUKD_QUERY_MORTON) && nq > 1) {
-    int32_t *perm = nullptr;
-    CKB_TRY(arena.alloc(&perm, nq));
-    CKB_TRY(morton_order_impl((const float *)d_queries, nq, L.D, nullptr, perm, st, mem));
-    s.q.order = perm;
+    CKB_TRY(query_order(d_queries, nq, CUKD_FLOAT32, L.D, nullptr, s.lo, s.hi, &s.q.order, st,
+                        &arena));
   }
   if (L.D == 2) return spatial::query_impl<2>(s, p->method, kind, st);
   if (L.D == 3) return spatial::query_impl<3>(s, p->method, kind, st);
