@@ -1169,6 +1169,119 @@ static int pow2ceil(int64_t v)
   return p;
 }
 
+// ---------------------------------------------------------------------------
+// trees of one tile: one launch, no scratch
+// ---------------------------------------------------------------------------
+// The general sequence takes four kernels, four fills and twenty allocations,
+// 69 us of host and launch time around 18 us of subtree work for 1000 points.
+// Here one CTA reads the keys from the records, finishes the tree in shared
+// memory and permutes the records in place, a word of each at a time.
+constexpr int kSmallThreads = 512;
+template <int D> struct SmallSmem {
+  SubSmem<D, kTile, kSmallThreads> sub;
+  uint16_t from[kTile];  // node -> input index
+};
+struct SmallArgs {
+  uint8_t *pts;
+  int n, stride, poff, doff, dshift;
+  uint32_t dmask;
+  uint32_t *worldBounds;
+};
+template <int SC, int D> struct SmallSrc {
+  const SmallArgs &a;
+  uint16_t *from;
+  template <class SM> __device__ void load(SM &S, int m) const
+  {
+    if (int(threadIdx.x) < D) {
+      S.rootLo[threadIdx.x] = 0xffffffffu;
+      S.rootHi[threadIdx.x] = 0u;
+    }
+    __syncthreads();
+    uint32_t lo[D], hi[D];
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+      lo[d] = 0xffffffffu;
+      hi[d] = 0u;
+    }
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+      const uint32_t *c = (const uint32_t *)(a.pts + int64_t(i) * a.stride + a.poff);
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        const uint32_t k = Scalar<SC>::key(c[d]);
+        S.key[d][i] = k;
+        lo[d] = min(lo[d], k);
+        hi[d] = max(hi[d], k);
+      }
+      S.idx[i] = uint32_t(i);
+    }
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+      const uint32_t l = __reduce_min_sync(0xffffffffu, lo[d]);
+      const uint32_t h = __reduce_max_sync(0xffffffffu, hi[d]);
+      if ((threadIdx.x & 31) == 0 && l <= h) {
+        atomicMin(&S.rootLo[d], l);
+        atomicMax(&S.rootHi[d], h);
+      }
+    }
+    __syncthreads();
+    if (a.worldBounds && int(threadIdx.x) < D) {
+      a.worldBounds[threadIdx.x] = Scalar<SC>::bits(S.rootLo[threadIdx.x]);
+      a.worldBounds[D + threadIdx.x] = Scalar<SC>::bits(S.rootHi[threadIdx.x]);
+    }
+  }
+  __device__ int anc_dim(int64_t) const { return 0; }  // the root has no ancestors
+  template <class SM> __device__ void settle(int64_t g, int, int piv, int, SM &) const
+  {
+    from[g] = uint16_t(piv);
+  }
+};
+
+template <int SC, int D>
+__global__ void __launch_bounds__(kSmallThreads) small_kernel(SmallArgs a)
+{
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  SmallSmem<D> &S = *reinterpret_cast<SmallSmem<D> *>(smem_raw);
+  SmallSrc<SC, D> src{a, S.from};
+  subtree_body<SC, D, kTile, kSmallThreads>(src, a.n, 0, 0, a.doff >= 0, S.sub);
+  __syncthreads();
+  constexpr int PER = kTile / kSmallThreads;
+  const int words = a.stride >> 2, dw = a.doff >= 0 ? a.doff >> 2 : -1;
+  for (int w = 0; w < words; w++) {
+    uint32_t v[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+      const int g = j * kSmallThreads + threadIdx.x;
+      v[j] = 0;
+      if (g < a.n) {
+        v[j] = ((const uint32_t *)(a.pts + int64_t(S.from[g]) * a.stride))[w];
+        if (w == dw)
+          v[j] = (v[j] & ~(a.dmask << a.dshift)) |
+                 ((uint32_t(S.sub.locDim[g]) & a.dmask) << a.dshift);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+      const int g = j * kSmallThreads + threadIdx.x;
+      if (g < a.n) ((uint32_t *)(a.pts + int64_t(g) * a.stride))[w] = v[j];
+    }
+    // the next word is read from places this one did not touch
+  }
+}
+
+template <int SC, int D>
+int build_small(void *pts, int64_t n, const Layout &L, void *worldBounds, cudaStream_t st)
+{
+  constexpr int smem = int(sizeof(SmallSmem<D>));
+  CKB_CUDA(cudaFuncSetAttribute(small_kernel<SC, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                smem));
+  SmallArgs a = {(uint8_t *)pts, int(n), L.stride, L.poff, L.doff, L.dshift, L.dmask,
+                 (uint32_t *)worldBounds};
+  small_kernel<SC, D><<<1, kSmallThreads, smem, st>>>(a);
+  CKB_CHECK_LAUNCH();
+  return CUKD_OK;
+}
+
 // The builder's launch sequence; Arena provides alloc(T **, count) -- the
 // caller's memory resource (TempArena) or the allocation-free builder's fixed
 // device scratch (StaticCarver) -- so both entry points run the same code.
@@ -1290,7 +1403,13 @@ template <int SC, int D>
 int build_impl(void *pts, int64_t n, const Layout &L, void *worldBounds, cudaStream_t st,
                const cukd_mem_resource *mem)
 {
+  if (n <= kTile) return build_small<SC, D>(pts, n, L, worldBounds, st);
   TempArena arena(st, mem);
+  // two key copies, candidates, permutation, dims, records; the rest is what
+  // a level's subtrees need
+  const size_t w = TempArena::rounded(sizeof(uint32_t) * n);
+  CKB_TRY(arena.reserve((3 * (D + 1) + 1) * w + TempArena::rounded(n) +
+                        TempArena::rounded(size_t(n) * L.stride) + TempArena::rounded(n) + 16384));
   return build_run<SC, D>(pts, n, L, worldBounds, st, arena);
 }
 
