@@ -598,5 +598,178 @@ __device__ __forceinline__ void knn_fast_one(const FastArgs &fa, int64_t myq, bo
   if (fa.status) fa.status[myq] = ok ? 0 : 1;
 }
 
+// FCP and k = 1 of one query: the same search (home subtree, one-word stack
+// entries, corner culling) for a single candidate, kept in registers with the
+// smallest distance bound of every other point seen.  The candidate is the
+// answer when everything else is farther: points seen by that bound, points
+// in culled boxes because boxes are culled above the candidate's bound (for
+// ints 16 ulps above, which covers the gap between L and the exact distance).
+// Whole calls, us, against the reference-order traversals (B200, 1M uniform
+// float3 queries, both sorted): 500K points 603 / 635 / 627 (stack-based,
+// stack-free, cct) -> 425; 64K 515 / 557 / 477 -> 377; 1000 299 / 364 / 281
+// -> 245; packed mixture records, 500K points 3326 / 4901 / 655 -> 475.
+template <int SC, int D, bool EXPL, bool VEC>
+__device__ __forceinline__ void fcp_fast_one(const FastArgs &fa, int64_t myq)
+{
+  using N = Num<SC>;
+  using T = typename N::T;
+  using E = typename N::E;
+  constexpr uint32_t SLACK = SC == 0 ? 0u : 16u;
+  constexpr int H = 3;
+  const query::QArgs &a = fa.q;
+  const query::TreeView tv = query::tree_of<D, 4>(a, myq);
+  const int n = int(tv.n);
+  const Nodes<SC, D, EXPL, VEC> nd(a, tv.tree);
+  T q[D];
+#pragma unroll
+  for (int d = 0; d < D; d++) q[d] = __ldg((const T *)a.queries + myq * D + d);
+  const E r2 = N::cutoff(a);
+  const bool usable = N::usable(r2);
+  uint32_t best = N::above(usable ? r2 : E(0)), second = ~0u;
+  int bestId = -1;
+  auto bound = [&](const T (&p)[D]) {
+    float s = N::sq(p[0], q[0]);
+#pragma unroll
+    for (int d = 1; d < D; d++) s = N::add(s, N::sq(p[d], q[d]));
+    return __float_as_uint(s);
+  };
+  auto sum = [](const float (&o)[D]) {
+    float s = o[0];
+#pragma unroll
+    for (int d = 1; d < D; d++) s = N::add(s, o[d]);
+    return __float_as_uint(s);
+  };
+  auto offer = [&](uint32_t l, int node) {
+    const bool nearer = l < best;
+    // (what a first candidate replaces is the cut-off, not a point)
+    second = umin(second, nearer ? (bestId >= 0 ? best : ~0u) : l);
+    best = nearer ? l : best;
+    bestId = nearer ? node : bestId;
+  };
+  int home = -1;
+  if (n > 0 && usable) {
+    home = 0;
+    const int lim = ((n + 1) >> (H - 1)) - 2;
+    int lvl = 0;
+#pragma unroll 1
+    for (;;) {
+      int dim;
+      const T c = nd.split(home, lvl, &dim);
+      T qc = q[0];
+#pragma unroll
+      for (int d = 1; d < D; d++) qc = d == dim ? q[d] : qc;
+      const int child = 2 * home + (qc < c ? 1 : 2);
+      if (child > lim) break;
+      home = child;
+      lvl++;
+    }
+    T p[D];
+    nd.point(home, p);
+    int node = home;
+#pragma unroll 1
+    for (uint32_t y = 2; node < n; y++) {
+      const int t = 31 - __clz(y);
+      const uint32_t next = ((uint32_t(home) + 1u) << t) - 1u + (y - (1u << t));
+      const uint32_t l = bound(p);
+      if (next < uint32_t(n)) nd.point(int(next), p);
+      offer(l, node);
+      node = int(next < uint32_t(n) ? next : uint32_t(n));
+    }
+  }
+  float off[D];
+  const T *bnd = (const T *)tv.bounds;
+#pragma unroll
+  for (int d = 0; d < D; d++) {
+    T v = q[d];
+    if (bnd) {
+      const T lo = __ldg(bnd + d), hi = __ldg(bnd + D + d);
+      v = v < lo ? lo : v;
+      v = hi < v ? hi : v;
+    }
+    off[d] = N::sq(v, q[d]);
+  }
+  // (stack entries as in knn_fast_one)
+  constexpr int FB = D == 2 ? 16 : (D == 3 ? 10 : 8);
+  constexpr uint32_t FM = (1u << FB) - 1u;
+  uint32_t offSt[32];
+  uint32_t trail = 0;
+  int sp = 0;
+  const uint32_t topBits = best + SLACK;
+  const bool scaled = topBits < 0x7f800000u && topBits > 0x0da24260u;  // > 1e-30
+  const uint32_t topExp = topBits >> 23;
+  const float scale = scaled ? __uint_as_float((253u + FB - topExp) << 23) : 0.f;
+  const float unit = scaled ? __uint_as_float((topExp + 1u - FB) << 23) : 0.f;
+  int curr = (home >= 0 && sum(off) <= topBits) ? 0 : n;
+  for (;;) {
+    if (curr >= n || curr == home) {
+      bool found = false;
+      while (trail) {
+        const uint32_t w = offSt[--sp];
+        const int lvl = 31 - __clz(trail);
+        trail ^= 1u << lvl;
+        float o[D];
+#pragma unroll
+        for (int d = 0; d < D; d++) o[d] = float((w >> (FB * d)) & FM) * unit;
+        if (sum(o) <= best + SLACK) {
+#pragma unroll
+          for (int d = 0; d < D; d++) off[d] = o[d];
+          const int c1 = curr + 1;
+          curr = ((c1 >> (31 - __clz(c1) - lvl)) ^ 1) - 1;
+          found = true;
+          break;
+        }
+      }
+      if (!found) break;
+    }
+    T p[D];
+    const int dim = nd.load(curr, p);
+    offer(bound(p), curr);
+    T nodeC = p[0], queryC = q[0];
+#pragma unroll
+    for (int d = 1; d < D; d++)
+      if (d == dim) {
+        nodeC = p[d];
+        queryC = q[d];
+      }
+    const bool leftIsClose = queryC < nodeC;
+    const int lChild = 2 * curr + 1;
+    const int farChild = leftIsClose ? lChild + 1 : lChild;
+    if (farChild < n) {
+      float fo[D];
+      const float split = N::sq(nodeC, queryC);
+#pragma unroll
+      for (int d = 0; d < D; d++) fo[d] = d == dim ? split : off[d];
+      if (sum(fo) <= best + SLACK) {
+        uint32_t w = 0;
+#pragma unroll
+        for (int d = 0; d < D; d++)
+          w |= (__float_as_uint(__fadd_rz(__fmul_rz(fo[d], scale), 8388608.f)) & FM) << (FB * d);
+        offSt[sp++] = w;
+        trail |= 2u << (31 - __clz(curr + 1));
+      }
+    }
+    curr = leftIsClose ? lChild : lChild + 1;
+  }
+  E X = r2;
+  bool ok = usable;
+  if (bestId >= 0) {
+    T p[D];
+    nd.point(bestId, p);
+    X = exact_d2<SC, D>(p, q);
+    ok = ok && X < r2 && N::above(X) < second;
+  } else if (!fa.fcp) {
+    // k = 1 takes a point at exactly the cut-off if the traversal visits it
+    ok = ok && N::above(r2) < second;
+  }
+  if (!ok) {
+    const int slot = atomicAdd(fa.fb_count, 1);
+    fa.fb_list[slot] = int32_t(myq);
+    return;
+  }
+  if (a.out_ids) a.out_ids[myq] = bestId;
+  if (a.out_d2) ((E *)a.out_d2)[myq] = X;
+  if (a.out_max) ((E *)a.out_max)[myq] = X;
+}
+
 }  // namespace fast
 }  // namespace ckb

@@ -245,12 +245,15 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
   const bool narrow = L.D <= kMaxFastDims;
   const bool exactOk = !visits && !a.heap_order && !(p->flags & CUKD_QUERY_REFERENCE_ORDER) &&
                        a.k <= 128 && narrow;
+  // The fast exact paths (see fast.cu): any visiting order, boundary-tie check,
+  // the queued queries a warp each, what that leaves in the reference order.
+  // A stack-free FCP or k = 1 with eps may return a point that is not the
+  // closest: only its own traversal says which.
+  const bool single = a.k == 1;
+  const bool fastOk = exactOk && !(single && p->method == CUKD_STACK_FREE && p->eps != 0.f);
   // few queries: a warp each (in any order, so without sorting them), and
-  // what it queues by the named traversal.  A stack-free FCP or k = 1 with
-  // eps may return a point that is not the closest: only its own traversal
-  // says which.
-  if (exactOk && nq <= warp_queries(L.scalar, a.k) &&
-      !(p->method == CUKD_STACK_FREE && p->eps != 0.f && a.k == 1)) {
+  // what it queues by the named traversal
+  if (fastOk && nq <= warp_queries(L.scalar, a.k)) {
     fast::WarpArgs wa = {};
     fast::FastArgs &fa = wa.f;
     fa.q = a;
@@ -291,16 +294,12 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     CKB_TRY(morton_order_impl((const float *)d_queries, nq, L.D, nullptr, perm, st, mem));
     a.order = perm;
   }
-  // fast exact path (see fast.cu): any visiting order, boundary-tie check,
-  // the queued queries a warp each, what that leaves in the reference order.
-  // (FCP and k = 1 stay on the reference traversals: with a single candidate
-  // the split-plane bound is already cheap and the corner bookkeeping does
-  // not pay for itself)
-  if (exactOk && knn && p->k >= 2) {
+  if (fastOk) {
     fast::WarpArgs wa = {};
     fast::FastArgs fa = {};
     fa.q = a;
     fa.kk = a.k;
+    fa.fcp = !knn;
     fa.method = p->method;
     int *ctr = nullptr;
     int32_t *lists = nullptr;
@@ -310,7 +309,7 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     fa.fb_count = ctr;
     fa.fb_list = lists;
     const bool packet = (p->flags & CUKD_QUERY_WARP_PACKET) && L.scalar == CUKD_FLOAT32 &&
-                        p->k <= 32;
+                        knn && !single && p->k <= 32;
     CKB_TRY(packet ? run_packet(fa, L.D, st) : run_fast(fa, L.scalar, L.D, st));
     wa.f = fa;
     wa.f.q.order = fa.fb_list;
