@@ -81,6 +81,22 @@ inline int64_t warp_queries(int scalar, int k)
 // and queued queries, of which the host does not know how many there are
 constexpr int kWarpQueue = 8192;
 
+// Whether visiting the queries in Z-order pays for sorting them: the sort is
+// 65 us of dependent launches and 14 us a million queries, and saves a
+// share of the search that grows with k, with D, and with a tree that the L2
+// does not hold.  Whole calls on random queries, us, sorted / not (B200,
+// float3, 10K points): FCP 500K 212 / 171; k = 4, 200K 213 / 151, 500K
+// 320 / 298; k = 16, 200K 330 / 284, 500K 542 / 580; k = 64, 50K 440 / 423,
+// 100K 635 / 706; record32, 4M points: FCP 500K 475 / 508, k = 16, 200K
+// 900 / 993.
+inline bool order_pays(int64_t nq, int k, int D, int64_t treeBytes)
+{
+  int64_t line = int64_t(6) << 20;
+  if (D >= 4) line /= 2;
+  if (treeBytes > (int64_t(96) << 20)) line /= 2;
+  return nq * (k == 1 ? 4 : k + 8) >= line;
+}
+
 // The warp-cooperative traversal (packet.cu): float kNN, k = 2..32, no
 // forest, no device-side query count.
 int run_packet(const fast::FastArgs &fa, int D, cudaStream_t st);

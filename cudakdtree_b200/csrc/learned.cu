@@ -721,10 +721,12 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   a.out_d2 = d_out_d2;
   a.visits = d_visits;
   a.block_size = p->block_size;
-  if ((p->flags & CUKD_QUERY_MORTON) && nq > 1 && d_world_bounds) {
+  if ((p->flags & CUKD_QUERY_MORTON) && !order_pays(nq, p->k, L.D, n * L.stride)) {
+    // (in the caller's order)
+  } else if ((p->flags & CUKD_QUERY_MORTON) && d_world_bounds) {
     CKB_TRY(query_order(d_queries, nq, L.scalar, L.D, d_world_bounds, nullptr, nullptr, &a.order,
                         st, &arena));
-  } else if ((p->flags & CUKD_QUERY_MORTON) && nq > 1 && L.scalar == CUKD_FLOAT32) {
+  } else if ((p->flags & CUKD_QUERY_MORTON) && L.scalar == CUKD_FLOAT32) {
     int32_t *perm = nullptr;
     CKB_TRY(arena.alloc(&perm, nq));
     CKB_TRY(cukd_morton_order((const float *)d_queries, nq, L.D, nullptr, perm, st, mem));

@@ -284,6 +284,8 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     CKB_TRY(run_tree_path(a, L.scalar, L.D, levels, codes, vals, st));
     CKB_TRY(radix_sort_pairs(codes, vals, codes2, vals2, nq, levels, st, &arena));
     a.order = (const int32_t *)vals;
+  } else if ((p->flags & CUKD_QUERY_MORTON) && fastOk && !order_pays(nq, a.k, L.D, n * L.stride)) {
+    // (in the caller's order)
   } else if ((p->flags & CUKD_QUERY_MORTON) && nq > 1 && narrow && d_world_bounds) {
     CKB_TRY(query_order(d_queries, nq, L.scalar, L.D, d_world_bounds, nullptr, nullptr, &a.order,
                         st, &arena));
