@@ -499,7 +499,13 @@ int cukd_batch_plan_create(cukd_batch_plan **out, int num_dims, int64_t num_clou
     p->poff.assign(1, 0);
     p->qoff.assign(1, 0);
   }
-  p->tuning.build_tile = 2048;
+  // Largest subtree of the shared-memory phase: 1024 points, whose CTAs are
+  // four to an SM, unless the clouds are too few to fill them (build and
+  // query, us, tiles of 1024 / 2048: 1024 clouds of 256..65536 points
+  // 3997 / 4238, 900 of 1025..2047 505 / 654; 200 clouds of 64..10000 points
+  // 401 / 367).
+  p->tuning.build_tile = h_point_offsets && num_clouds > 0 &&
+                                 h_point_offsets[num_clouds] < (int64_t(1) << 19) ? 2048 : 1024;
   p->tuning.block_size = 128;
   p->tuning.queries_per_thread = 1;
   p->tuning.morton = 1;
