@@ -1,13 +1,15 @@
 // Whole-batch FCP / kNN queries over a left-balanced k-d tree (sm_100a).
 //
-// One thread runs one query with exactly the reference's control flow --
+// These are the reference-order kernels; most calls are answered by the fast
+// exact paths (fast.cu, warp.cuh) and leave them the ties whose outcome depends
+// on the order.  One thread runs one query with the reference's control flow --
 // traverse_default (traverse-default-stack-based.h:24-108),
 // traverse_stack_free (traverse-stack-free.h:24-117) and traverse_cct
 // (traverse-cct.h:25-99) -- so candidates reach the result object in the
 // same order and the answers are bit-identical, ties included.  What is
 // B200-specific is around that core:
-//   - queries are visited in 30-bit Morton order (morton.cu) so a warp's
-//     32 traversals walk nearby paths, and results are scattered back;
+//   - queries are visited in Morton order (morton.cu) where that pays, so a
+//     warp's 32 traversals walk nearby paths, and results are scattered back;
 //   - node records are read through the read-only path (__ldg), 16-byte
 //     vector loads for 16-byte records;
 //   - fixed-size candidate lists live in registers with an early-out

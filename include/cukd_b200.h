@@ -194,8 +194,9 @@ typedef enum cukd_method {
 } cukd_method;
 
 enum {
-  /* sort queries along a 30-bit Morton curve before traversal and scatter
-   * results back to the caller's order (results are unchanged) */
+  /* visit the queries along a Morton curve where sorting them pays (by their
+   * number, k, the dimension and the tree's size) and scatter the results
+   * back to the caller's order (results are unchanged) */
   CUKD_QUERY_MORTON = 1,
   /* kNN: return the candidate list in the reference HeapCandidateList's
    * heap order instead of ascending (d2, id) order */
