@@ -250,12 +250,14 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
   // The fast exact paths (see fast.cu): any visiting order, boundary-tie check,
   // the queued queries a warp each, what that leaves in the reference order.
   // A stack-free FCP or k = 1 with eps may return a point that is not the
-  // closest: only its own traversal says which.
+  // closest: only its own traversal says which.  Lists ignore eps but for
+  // ties, which the warp kernel cannot tell from their last point alone.
   const bool single = a.k == 1;
-  const bool fastOk = exactOk && !(single && p->method == CUKD_STACK_FREE && p->eps != 0.f);
+  const bool plain = !(p->method == CUKD_STACK_FREE && p->eps != 0.f);
+  const bool fastOk = exactOk && (plain || !single);
   // few queries: a warp each (in any order, so without sorting them), and
   // what it queues by the named traversal
-  if (fastOk && nq <= warp_queries(L.scalar, a.k)) {
+  if (fastOk && plain && nq <= warp_queries(L.scalar, a.k)) {
     fast::WarpArgs wa = {};
     fast::FastArgs &fa = wa.f;
     fa.q = a;

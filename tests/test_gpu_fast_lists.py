@@ -5,6 +5,7 @@ that leave lists unfilled, records that can and cannot be read as vectors,
 tie-heavy and duplicate points.  Bit-exact: the reference-order kernels are
 pinned to the oracle in test_gpu_query.py.
 """
+import ctypes as C
 import math
 
 import pytest
@@ -100,3 +101,21 @@ def test_far_queries_keep_many_subtrees_pending():
     q = torch.randn((300, 3), device="cuda", generator=g) * 1e-3
     for k in (1, 16, 100):
         _check(tree, q, k, "cct", None, wb)
+
+
+@pytest.mark.parametrize("nq", [300, 17000])
+@pytest.mark.parametrize("k", [2, 8])
+def test_stack_free_eps_does_not_change_lists(nq, k):
+    """eps of a stack-free kNN applies to ties only: without ties the list is
+    the exact one, for few queries as for many."""
+    tree = torch.from_numpy(make_points(20000, 3, "uniform", seed=9)).cuda()
+    wb = ck.build_tree(tree)
+    lay = ck.infer_layout(tree)
+    q = torch.from_numpy(make_queries(nq, 3, "uniform", seed=10)).cuda()
+    want = ck.knn(tree, q, k, "stack_free", world_bounds=wb)
+    p = ck._params("stack_free", k, eps=0.5)
+    ids, d2 = torch.empty_like(want[0]), torch.empty_like(want[1])
+    ck._check(ck.lib().cukd_knn(ck._ptr(tree), 20000, C.byref(lay), ck._ptr(wb), ck._ptr(q), nq,
+                                C.byref(p), ck._ptr(ids), ck._ptr(d2), None, ck._stream(None),
+                                None), "cukd_knn")
+    assert torch.equal(ids, want[0]) and torch.equal(d2, want[1])
