@@ -259,7 +259,12 @@ __global__ void root_kernel(BuildBufs b, uint32_t n, uint32_t threshold)
   *b.st = s;
 }
 
-// selectSplits (:316-396): the widest extent's centre; dim -1: degenerate
+// selectSplits (:316-396): the widest extent's centre; dim -1: degenerate.
+// Degenerate is every centre that is not inside its box: one that rounds onto
+// a face, and the infinite or NaN centre of a box whose l + h overflows or
+// that holds infinities of both signs or a NaN.  Such a centre leaves one side
+// empty and the other as it was, level after level; the alternating split
+// halves the prims instead, so both children of every split hold some.
 template <int D>
 __device__ inline int decide(const int32_t *lo, const int32_t *hi, float *pos)
 {
@@ -273,7 +278,7 @@ __device__ inline int decide(const int32_t *lo, const int32_t *hi, float *pos)
     widestWidth = width;
     dim = d;
     at = __fmul_rn(0.5f, __fadd_rn(l, h));
-    if (at == l || at == h) dim = -2 - d;  // rounds onto the box
+    if (!(at > l && at < h)) dim = -2 - d;
   }
   if (dim < 0) {
     dim = -1;

@@ -582,8 +582,11 @@ int cko_spatial_build(int D, const float *coords, int64_t n, int leaf_threshold,
       }
       float pos = 0.f;
       if (widestDim >= 0) {
+        /* degenerate: a centre that rounds onto a face, or one that is
+         * infinite or NaN (l + h overflows, infinities, NaN), which would
+         * leave one side empty for ever */
         pos = 0.5f * (abox_decode(in->lo[widestDim]) + abox_decode(in->hi[widestDim]));
-        if (pos == abox_decode(in->lo[widestDim]) || pos == abox_decode(in->hi[widestDim]))
+        if (!(pos > abox_decode(in->lo[widestDim]) && pos < abox_decode(in->hi[widestDim])))
           widestDim = -1;
       }
       if (widestDim < 0) pos = abox_decode(in->lo[0]);
