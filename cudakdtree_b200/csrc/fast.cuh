@@ -73,9 +73,12 @@ int run_warp(const fast::WarpArgs &wa, int scalar, int D, cudaStream_t st);
 // warp per query (B200, uniform float3, 100K points): k = 8, 1000 queries
 // 157 / 41, 16384 175 / 117, 32768 181 / 200; k = 32, 16384 257 / 206; k = 64,
 // 8192 367 / 295, 16384 361 / 530; int3, 1M points, k = 16, 8192 146 / 122,
-// 16384 146 / 198.
+// 16384 146 / 198.  FCP and k = 1 (FCP, 500K points): 4000 queries 61 / 47,
+// 8000 62 / 64, 16000 63 / 85; with ties, which the thread kernel has to
+// settle after the warp kernel, 1000 64 / 92.
 inline int64_t warp_queries(int scalar, int k)
 {
+  if (k == 1) return 6144;
   return scalar == CUKD_FLOAT32 && k <= 32 ? 16384 : 8192;
 }
 // and queued queries, of which the host does not know how many there are

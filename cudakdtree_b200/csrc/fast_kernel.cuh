@@ -51,23 +51,33 @@ int launch_fast(const FastArgs &fa, cudaStream_t st)
   return CUKD_OK;
 }
 
-template <int SC, int D, bool EXPL, bool VEC>
+template <int SC, int D, bool EXPL, bool VEC, bool FCP>
 __global__ void __launch_bounds__(128, 10) fcp_fast_kernel(const __grid_constant__ FastArgs fa)
 {
-  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i < fa.q.nq) fcp_fast_one<SC, D, EXPL, VEC>(fa, fa.q.order ? int64_t(fa.q.order[i]) : i);
+  const int64_t limit = fa.q.count_ptr ? int64_t(*fa.q.count_ptr) : fa.q.nq;
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < limit;
+       i += int64_t(gridDim.x) * blockDim.x)
+    fcp_fast_one<SC, D, EXPL, VEC, FCP>(fa, fa.q.order ? int64_t(fa.q.order[i]) : i);
+}
+
+template <int SC, int D, bool EXPL, bool VEC, bool FCP>
+int launch_fcp(const FastArgs &fa, cudaStream_t st)
+{
+  const int bs = fa.q.block_size > 0 ? std::min(fa.q.block_size, 128) : 128;
+  int64_t grid = div_up(fa.q.nq, bs);
+  if (fa.q.count_ptr) grid = std::min<int64_t>(grid, int64_t(kNumSMs) * 10);
+  fcp_fast_kernel<SC, D, EXPL, VEC, FCP><<<unsigned(grid), bs, 0, st>>>(fa);
+  CKB_CHECK_LAUNCH();
+  return CUKD_OK;
 }
 
 template <int SC, int D, bool EXPL, bool VEC>
 int dispatch_kc(const FastArgs &fa, cudaStream_t st)
 {
   const int slots = fa.kk + 1;
-  if (slots == 2) {  // FCP or k = 1, without a queue or seeds
-    const int bs = fa.q.block_size > 0 ? std::min(fa.q.block_size, 128) : 128;
-    fcp_fast_kernel<SC, D, EXPL, VEC><<<unsigned(div_up(fa.q.nq, bs)), bs, 0, st>>>(fa);
-    CKB_CHECK_LAUNCH();
-    return CUKD_OK;
-  }
+  if (slots == 2)  // without seeds
+    return fa.fcp ? launch_fcp<SC, D, EXPL, VEC, true>(fa, st)
+                  : launch_fcp<SC, D, EXPL, VEC, false>(fa, st);
   if (slots <= 5) return launch_fast<SC, D, EXPL, VEC, 5>(fa, st);
   if (slots <= 9) return launch_fast<SC, D, EXPL, VEC, 9>(fa, st);
   if (slots <= 17) return launch_fast<SC, D, EXPL, VEC, 17>(fa, st);

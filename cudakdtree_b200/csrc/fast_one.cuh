@@ -161,16 +161,29 @@ __device__ __forceinline__ typename Num<SC>::E exact_d2(const typename Num<SC>::
   return s;
 }
 
+// Which side of a split the traversal `method` takes first: the left one for a
+// query strictly left of the plane (stack-based, cct) or not right of it
+// (stack-free).
+template <class T> __device__ __forceinline__ bool left_first(int method, T qc, T c)
+{
+  return method == CUKD_STACK_FREE ? !(qc > c) : qc < c;
+}
+
 // Whether the reference's traversal `method` visits `node` whatever its
 // candidate list holds meanwhile, X being the final k-th distance: its list's
 // cull distance never drops below X, and it skips a child only on the far
 // side, when the child's plane (cct: box) distance is not below the cull
 // distance.  So a node is visited for sure when every far-side step on its
 // path has a distance below X.
+//
+// For a single candidate (FCP, k = 1) the cull distance is above X until the
+// first point at distance X is visited, and X from then on.  With that point
+// in `first`, a far side at distance X is entered exactly when it holds
+// `first`, and the outcome is exact: the node is visited, or it is not.
 template <int SC, int D, bool EXPL, bool VEC>
 __device__ __forceinline__ bool surely_visited(const FastArgs &fa, const Nodes<SC, D, EXPL, VEC> &nd,
                                const typename Num<SC>::T (&q)[D], const void *bounds, int node,
-                               typename Num<SC>::E X)
+                               typename Num<SC>::E X, int first = -1)
 {
   using N = Num<SC>;
   using T = typename N::T;
@@ -186,27 +199,26 @@ __device__ __forceinline__ bool surely_visited(const FastArgs &fa, const Nodes<S
       close[d] = v;
     }
   }
-  const int depth = level_of(node);
+  const int depth = level_of(node), firstDepth = first < 0 ? -1 : level_of(first);
 #pragma unroll 1
   for (int lvl = 0; lvl < depth; lvl++) {
     const int a = ((node + 1) >> (depth - lvl)) - 1;
-    const bool isLeft = (((node + 1) >> (depth - lvl - 1)) & 1) == 0;
+    const int child = (node + 1) >> (depth - lvl - 1);  // (+ 1)
     int dim;
     const T c = nd.split(a, lvl, &dim);
     T qc = q[0];
 #pragma unroll
     for (int d = 1; d < D; d++) qc = d == dim ? q[d] : qc;
+    if (((child & 1) == 0) == left_first(fa.method, qc, c)) continue;  // the near side
+    bool in;
     if (fa.method == CUKD_CCT) {
-      if (isLeft == (qc < c)) continue;  // the near side
 #pragma unroll
       for (int d = 0; d < D; d++) close[d] = d == dim ? c : close[d];
-      if (!(exact_d2<SC, D>(close, q) < X)) return false;
+      in = exact_d2<SC, D>(close, q) < X;
     } else {
-      // near only when strictly on that side (the two plane-culling
-      // traversals differ in where they count a query on the plane)
-      if (isLeft ? qc < c : qc > c) continue;
-      if (!(N::exact_sq(qc, c) < X)) return false;
+      in = N::exact_sq(qc, c) < X;
     }
+    if (!in && (firstDepth <= lvl || ((first + 1) >> (firstDepth - lvl - 1)) != child)) return false;
   }
   return true;
 }
@@ -599,22 +611,35 @@ __device__ __forceinline__ void knn_fast_one(const FastArgs &fa, int64_t myq, bo
 }
 
 // FCP and k = 1 of one query: the same search (home subtree, one-word stack
-// entries, corner culling) for a single candidate, kept in registers with the
-// smallest distance bound of every other point seen.  The candidate is the
-// answer when everything else is farther: points seen by that bound, points
-// in culled boxes because boxes are culled above the candidate's bound (for
-// ints 16 ulps above, which covers the gap between L and the exact distance).
-// Whole calls, us, against the reference-order traversals (B200, 1M uniform
-// float3 queries, both sorted): 500K points 603 / 635 / 627 (stack-based,
-// stack-free, cct) -> 425; 64K 515 / 557 / 477 -> 377; 1000 299 / 364 / 281
-// -> 245; packed mixture records, 500K points 3326 / 4901 / 655 -> 475.
-template <int SC, int D, bool EXPL, bool VEC>
+// entries, corner culling) for a single candidate in registers, with the
+// reference's answer at ties:
+//   - FCP keeps the first visited of the points at the smallest distance X.
+//     Until then the reference's cull distance is above X, so that point is
+//     the first in the traversal's preorder (near side before far side).
+//     This search leaves preorder only for the home subtree: that lies on the
+//     near path, so its points and the path's above it come before all others
+//     and are compared by preorder; later ones have to be strictly nearer.
+//   - k = 1 keeps the smallest id of the points at distance X that the
+//     reference visits: the smallest seen here, if `surely_visited` (exact,
+//     given the first one in preorder) says so; else the query is queued.
+//     Far sides that the reference cannot enter are not entered.
+// Boxes beyond `top` are culled, which is the bound of the candidate's
+// distance (rounded up for ints, whose bound L is rounded down); boxes at it
+// only where a point there can matter, so a group of points at the nearest
+// distance costs a path (FCP), or what the reference itself visits of it.
+//
+// Whole calls of 1M float3 queries, us, stack-based reference order (sorted) ->
+// FCP here / k = 1 here (B200): 1M uniform points 619 -> 394 / 413; with ties,
+// cell centres of a 100^3 lattice 762 -> 498 / 658 and its half steps
+// 704 -> 423 / 668, 500K points twice each 212 -> 140 / 160, 15K points 64
+// times each from elsewhere 4780 -> 3060 / 3390 (these five, when ties were
+// left to the reference order after this search: -, 1508, 1163, 312, 6750).
+template <int SC, int D, bool EXPL, bool VEC, bool FCP>
 __device__ __forceinline__ void fcp_fast_one(const FastArgs &fa, int64_t myq)
 {
   using N = Num<SC>;
   using T = typename N::T;
   using E = typename N::E;
-  constexpr uint32_t SLACK = SC == 0 ? 0u : 16u;
   constexpr int H = 3;
   const query::QArgs &a = fa.q;
   const query::TreeView tv = query::tree_of<D, 4>(a, myq);
@@ -623,10 +648,12 @@ __device__ __forceinline__ void fcp_fast_one(const FastArgs &fa, int64_t myq)
   T q[D];
 #pragma unroll
   for (int d = 0; d < D; d++) q[d] = __ldg((const T *)a.queries + myq * D + d);
-  const E r2 = N::cutoff(a);
-  const bool usable = N::usable(r2);
-  uint32_t best = N::above(usable ? r2 : E(0)), second = ~0u;
-  int bestId = -1;
+  // the nearest distance so far (at first the cut-off, at which k = 1 still
+  // takes points and FCP does not), the first point at it in preorder, and
+  // (k = 1) the smallest id seen at it
+  E bestD = N::cutoff(a);
+  uint32_t top = N::above(bestD);
+  int first = -1, least = -1;
   auto bound = [&](const T (&p)[D]) {
     float s = N::sq(p[0], q[0]);
 #pragma unroll
@@ -639,15 +666,44 @@ __device__ __forceinline__ void fcp_fast_one(const FastArgs &fa, int64_t myq)
     for (int d = 1; d < D; d++) s = N::add(s, o[d]);
     return __float_as_uint(s);
   };
-  auto offer = [&](uint32_t l, int node) {
-    const bool nearer = l < best;
-    // (what a first candidate replaces is the cut-off, not a point)
-    second = umin(second, nearer ? (bestId >= 0 ? best : ~0u) : l);
-    best = nearer ? l : best;
-    bestId = nearer ? node : bestId;
+  auto coord = [&](int dim) {
+    T qc = q[0];
+#pragma unroll
+    for (int d = 1; d < D; d++) qc = d == dim ? q[d] : qc;
+    return qc;
+  };
+  auto precedes = [&](int x, int y) {  // in preorder, x != y
+    const int lx = level_of(x), ly = level_of(y), m = lx < ly ? lx : ly;
+    const uint32_t ax = uint32_t(x + 1) >> (lx - m), ay = uint32_t(y + 1) >> (ly - m);
+    if (ax == ay) return lx < ly;
+    const int s = 32 - __clz(ax ^ ay);  // up to their last common ancestor
+    int dim;
+    const T c = nd.split(int(ax >> s) - 1, m - s, &dim);
+    return (((ax >> (s - 1)) & 1u) == 0) == left_first(fa.method, coord(dim), c);
+  };
+  // early: in the home subtree or on the path to it
+  auto offer = [&](const T (&p)[D], int node, bool early) {
+    const uint32_t l = bound(p);
+    if (SC == 0 && FCP) {  // l is the distance: no branch but at early ties
+      const bool tie = early && l == top;
+      const bool nearer = l < top;
+      top = nearer ? l : top;
+      first = nearer ? node : first;
+      if (tie && first >= 0 && precedes(node, first)) first = node;
+    } else if (l <= top) {
+      const E d = exact_d2<SC, D>(p, q);
+      if (d < bestD) {
+        bestD = d;
+        top = N::above(d);
+        first = least = node;
+      } else if (d == bestD && (early || !FCP)) {
+        if (early && first >= 0 && precedes(node, first)) first = node;
+        least = int(umin(uint32_t(least), uint32_t(node)));
+      }
+    }
   };
   int home = -1;
-  if (n > 0 && usable) {
+  if (n > 0) {
     home = 0;
     const int lim = ((n + 1) >> (H - 1)) - 2;
     int lvl = 0;
@@ -655,10 +711,7 @@ __device__ __forceinline__ void fcp_fast_one(const FastArgs &fa, int64_t myq)
     for (;;) {
       int dim;
       const T c = nd.split(home, lvl, &dim);
-      T qc = q[0];
-#pragma unroll
-      for (int d = 1; d < D; d++) qc = d == dim ? q[d] : qc;
-      const int child = 2 * home + (qc < c ? 1 : 2);
+      const int child = 2 * home + (left_first(fa.method, coord(dim), c) ? 1 : 2);
       if (child > lim) break;
       home = child;
       lvl++;
@@ -670,9 +723,11 @@ __device__ __forceinline__ void fcp_fast_one(const FastArgs &fa, int64_t myq)
     for (uint32_t y = 2; node < n; y++) {
       const int t = 31 - __clz(y);
       const uint32_t next = ((uint32_t(home) + 1u) << t) - 1u + (y - (1u << t));
-      const uint32_t l = bound(p);
+      T c[D];
+#pragma unroll
+      for (int d = 0; d < D; d++) c[d] = p[d];
       if (next < uint32_t(n)) nd.point(int(next), p);
-      offer(l, node);
+      offer(c, node, true);
       node = int(next < uint32_t(n) ? next : uint32_t(n));
     }
   }
@@ -694,36 +749,15 @@ __device__ __forceinline__ void fcp_fast_one(const FastArgs &fa, int64_t myq)
   uint32_t offSt[32];
   uint32_t trail = 0;
   int sp = 0;
-  const uint32_t topBits = best + SLACK;
-  const bool scaled = topBits < 0x7f800000u && topBits > 0x0da24260u;  // > 1e-30
-  const uint32_t topExp = topBits >> 23;
+  const bool scaled = top < 0x7f800000u && top > 0x0da24260u;  // > 1e-30
+  const uint32_t topExp = top >> 23;
   const float scale = scaled ? __uint_as_float((253u + FB - topExp) << 23) : 0.f;
   const float unit = scaled ? __uint_as_float((topExp + 1u - FB) << 23) : 0.f;
-  int curr = (home >= 0 && sum(off) <= topBits) ? 0 : n;
-  for (;;) {
-    if (curr >= n || curr == home) {
-      bool found = false;
-      while (trail) {
-        const uint32_t w = offSt[--sp];
-        const int lvl = 31 - __clz(trail);
-        trail ^= 1u << lvl;
-        float o[D];
-#pragma unroll
-        for (int d = 0; d < D; d++) o[d] = float((w >> (FB * d)) & FM) * unit;
-        if (sum(o) <= best + SLACK) {
-#pragma unroll
-          for (int d = 0; d < D; d++) off[d] = o[d];
-          const int c1 = curr + 1;
-          curr = ((c1 >> (31 - __clz(c1) - lvl)) ^ 1) - 1;
-          found = true;
-          break;
-        }
-      }
-      if (!found) break;
-    }
+  int curr = 0;
+  auto step = [&](bool early) {  // visits curr and goes on to its near child
     T p[D];
     const int dim = nd.load(curr, p);
-    offer(bound(p), curr);
+    offer(p, curr, early);
     T nodeC = p[0], queryC = q[0];
 #pragma unroll
     for (int d = 1; d < D; d++)
@@ -731,7 +765,7 @@ __device__ __forceinline__ void fcp_fast_one(const FastArgs &fa, int64_t myq)
         nodeC = p[d];
         queryC = q[d];
       }
-    const bool leftIsClose = queryC < nodeC;
+    const bool leftIsClose = left_first(fa.method, queryC, nodeC);
     const int lChild = 2 * curr + 1;
     const int farChild = leftIsClose ? lChild + 1 : lChild;
     if (farChild < n) {
@@ -739,36 +773,62 @@ __device__ __forceinline__ void fcp_fast_one(const FastArgs &fa, int64_t myq)
       const float split = N::sq(nodeC, queryC);
 #pragma unroll
       for (int d = 0; d < D; d++) fo[d] = d == dim ? split : off[d];
-      if (sum(fo) <= best + SLACK) {
+      // (k = 1: a box at `top` may hold a point that counts, if the
+      // reference enters it, which cct does by the box, the others by the plane)
+      const uint32_t box = sum(fo);
+      if (FCP ? box < top : box <= top) {
+        const bool enter = FCP || box < top ||
+                           (fa.method != CUKD_CCT && __float_as_uint(split) < top);
         uint32_t w = 0;
 #pragma unroll
         for (int d = 0; d < D; d++)
           w |= (__float_as_uint(__fadd_rz(__fmul_rz(fo[d], scale), 8388608.f)) & FM) << (FB * d);
-        offSt[sp++] = w;
-        trail |= 2u << (31 - __clz(curr + 1));
+        offSt[sp] = w;
+        sp += int(enter);
+        trail |= (enter ? 2u : 0u) << (31 - __clz(curr + 1));
       }
     }
     curr = leftIsClose ? lChild : lChild + 1;
+  };
+  auto pop = [&]() {  // curr: the last pending far child that still matters
+    while (trail) {
+      const uint32_t w = offSt[--sp];
+      const int lvl = 31 - __clz(trail);
+      trail ^= 1u << lvl;
+      float o[D];
+#pragma unroll
+      for (int d = 0; d < D; d++) o[d] = float((w >> (FB * d)) & FM) * unit;
+      if (FCP ? sum(o) < top : sum(o) <= top) {
+#pragma unroll
+        for (int d = 0; d < D; d++) off[d] = o[d];
+        const int c1 = curr + 1;
+        curr = ((c1 >> (31 - __clz(c1) - lvl)) ^ 1) - 1;
+        return true;
+      }
+    }
+    return false;
+  };
+  if (n > 0 && sum(off) <= top) {
+    // the path to the home subtree, then what is pending
+    while (curr < home) step(true);
+    bool more = pop();
+    while (more) {
+      step(false);
+      if (curr >= n) more = pop();
+    }
   }
-  E X = r2;
-  bool ok = usable;
-  if (bestId >= 0) {
-    T p[D];
-    nd.point(bestId, p);
-    X = exact_d2<SC, D>(p, q);
-    ok = ok && X < r2 && N::above(X) < second;
-  } else if (!fa.fcp) {
-    // k = 1 takes a point at exactly the cut-off if the traversal visits it
-    ok = ok && N::above(r2) < second;
+  if (SC == 0 && FCP) {  // (of the same four bytes)
+    const float d = __uint_as_float(top);
+    memcpy(&bestD, &d, 4);
   }
-  if (!ok) {
-    const int slot = atomicAdd(fa.fb_count, 1);
-    fa.fb_list[slot] = int32_t(myq);
+  if (!FCP && least != first &&
+      !surely_visited<SC, D, EXPL, VEC>(fa, nd, q, tv.bounds, least, bestD, first)) {
+    fa.fb_list[atomicAdd(fa.fb_count, 1)] = int32_t(myq);
     return;
   }
-  if (a.out_ids) a.out_ids[myq] = bestId;
-  if (a.out_d2) ((E *)a.out_d2)[myq] = X;
-  if (a.out_max) ((E *)a.out_max)[myq] = X;
+  if (a.out_ids) a.out_ids[myq] = FCP ? first : least;
+  if (a.out_d2) ((E *)a.out_d2)[myq] = bestD;
+  if (a.out_max) ((E *)a.out_max)[myq] = bestD;
 }
 
 }  // namespace fast

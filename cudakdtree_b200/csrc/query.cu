@@ -249,12 +249,15 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
                        a.k <= 128 && narrow;
   // The fast exact paths (see fast.cu): any visiting order, boundary-tie check,
   // the queued queries a warp each, what that leaves in the reference order.
-  // A stack-free FCP or k = 1 with eps may return a point that is not the
-  // closest: only its own traversal says which.  Lists ignore eps but for
-  // ties, which the warp kernel cannot tell from their last point alone.
+  // FCP and k = 1 have a search that knows ties, too (fcp_fast_one); one that
+  // is stack-free with eps may return a point that is not the closest, and
+  // one with a NaN or negative cut-off what its traversal makes of that: both
+  // are left to their traversal.  Lists ignore eps but for ties, which the
+  // warp kernel cannot tell from their last point alone.
   const bool single = a.k == 1;
   const bool plain = !(p->method == CUKD_STACK_FREE && p->eps != 0.f);
-  const bool fastOk = exactOk && (plain || !single);
+  const bool usable = L.scalar == CUKD_FLOAT32 ? a.cutoff == a.cutoff : a.cutoff_d2 >= 0;
+  const bool fastOk = exactOk && (!single || (plain && usable));
   // few queries: a warp each (in any order, so without sorting them), and
   // what it queues by the named traversal
   if (fastOk && plain && nq <= warp_queries(L.scalar, a.k)) {
@@ -264,19 +267,28 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     fa.kk = a.k;
     fa.fcp = !knn;
     fa.method = p->method;
-    int *queue = nullptr;  // its length, then the queries
-    CKB_TRY(arena.alloc(&queue, nq + 1));
-    CKB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), st));
+    int *queue = nullptr;  // the lengths of two, then their queries
+    const bool two = single && knn;
+    CKB_TRY(arena.alloc(&queue, two ? 2 * nq + 2 : nq + 2));
+    CKB_CUDA(cudaMemsetAsync(queue, 0, 2 * sizeof(int), st));
     fa.fb_count = queue;
-    fa.fb_list = queue + 1;
+    fa.fb_list = queue + 2;
     CKB_TRY(run_warp(wa, L.scalar, L.D, st));
-    if (p->d_reordered_count)
-      CKB_CUDA(cudaMemcpyAsync(p->d_reordered_count, fa.fb_count, sizeof(int),
-                               cudaMemcpyDeviceToDevice, st));
     QArgs b = a;
     b.order = fa.fb_list;
     b.count_ptr = fa.fb_count;
-    return run_query(b, L.scalar, L.D, p->method, kind, st);
+    if (single) {  // ties by the thread kernel, which leaves none of FCP
+      fa.q = b;
+      fa.fb_count = queue + 1;
+      fa.fb_list = queue + 2 + nq;
+      CKB_TRY(run_fast(fa, L.scalar, L.D, st));
+      b.order = fa.fb_list;
+      b.count_ptr = fa.fb_count;
+    }
+    if (p->d_reordered_count)
+      CKB_CUDA(cudaMemcpyAsync(p->d_reordered_count, b.count_ptr, sizeof(int),
+                               cudaMemcpyDeviceToDevice, st));
+    return !knn ? CUKD_OK : run_query(b, L.scalar, L.D, p->method, kind, st);
   }
   if ((p->flags & CUKD_QUERY_TREE_ORDER) && nq > 1 && n > 0 && narrow) {
     uint32_t *codes = nullptr, *codes2 = nullptr, *vals = nullptr, *vals2 = nullptr;
@@ -300,12 +312,32 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     CKB_TRY(morton_order_impl((const float *)d_queries, nq, L.D, nullptr, perm, st, mem));
     a.order = perm;
   }
+  if (fastOk && single) {
+    fast::FastArgs fa = {};
+    fa.q = a;
+    fa.kk = 1;
+    fa.fcp = !knn;
+    fa.method = p->method;
+    int *queue = nullptr;  // its length, then the queries (of FCP none)
+    CKB_TRY(arena.alloc(&queue, knn ? nq + 1 : 1));
+    if (knn || p->d_reordered_count) CKB_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), st));
+    fa.fb_count = queue;
+    fa.fb_list = queue + 1;
+    CKB_TRY(run_fast(fa, L.scalar, L.D, st));
+    if (p->d_reordered_count)
+      CKB_CUDA(cudaMemcpyAsync(p->d_reordered_count, queue, sizeof(int), cudaMemcpyDeviceToDevice,
+                               st));
+    QArgs b = a;
+    b.order = fa.fb_list;
+    b.count_ptr = fa.fb_count;
+    return !knn ? CUKD_OK : run_query(b, L.scalar, L.D, p->method, kind, st);
+  }
   if (fastOk) {
     fast::WarpArgs wa = {};
     fast::FastArgs fa = {};
     fa.q = a;
     fa.kk = a.k;
-    fa.fcp = !knn;
+    fa.fcp = false;
     fa.method = p->method;
     int *ctr = nullptr;
     int32_t *lists = nullptr;
@@ -315,7 +347,7 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     fa.fb_count = ctr;
     fa.fb_list = lists;
     const bool packet = (p->flags & CUKD_QUERY_WARP_PACKET) && L.scalar == CUKD_FLOAT32 &&
-                        knn && !single && p->k <= 32;
+                        p->k <= 32;
     CKB_TRY(packet ? run_packet(fa, L.D, st) : run_fast(fa, L.scalar, L.D, st));
     wa.f = fa;
     wa.f.q.order = fa.fb_list;

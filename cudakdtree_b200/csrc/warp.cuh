@@ -117,7 +117,13 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     }
   }
   const int k = fa.kk;
-  const int K = fa.fcp ? 2 : k;  // keys that count (FCP: the second tells a tie)
+  // keys that count; for FCP and k = 1 the second tells a tie, and once there
+  // are two, boxes at the second's distance are of use only to k = 1, to find
+  // the smallest id of the tied points (while they are at most kTied: a group
+  // of equal points may be the whole tree)
+  constexpr int kTied = 32;
+  const bool single = k == 1;
+  const int K = single ? 2 : k;
   // this lane's place in a treelet (lane 31 has none)
   const int t = 31 - __clz(lane + 1);
   for (int64_t w = blockIdx.x * int64_t(kWarpsPerBlock) + wid; w < limit;
@@ -134,14 +140,16 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     L list;
     list.init(r2);
     auto kth = list.key[0];
-    uint32_t cull = N::above(r2);
+    int tied = 0;  // points seen at the first key's distance
+    uint32_t cull = N::above(r2) + 1u;  // boxes at this distance and more are skipped
     auto refresh = [&]() {
 #pragma unroll
       for (int i = 0; i < KL; i++) {
         const auto v = L::shfl(list.key[i], (K - 1) & 31);
         if (i == (K - 1) >> 5) kth = v;
       }
-      cull = N::above(L::d2(kth));
+      const bool exclusive = single && L::id(kth) != -1 && (fa.fcp || tied > kTied);
+      cull = N::above(L::d2(kth)) + (exclusive ? 0u : 1u);
     };
     auto insert = [&](auto x) {
 #pragma unroll
@@ -216,7 +224,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
       float off[D];
 #pragma unroll
       for (int d = 0; d < D; d++) off[d] = rootOff[d];
-      if (sum(off) > cull) break;
+      if (sum(off) >= cull) break;
       for (;;) {
         const int lvl = level_of(curr);
         const int h = lvl == 0 ? rootLevels : kTreelet;
@@ -254,17 +262,24 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
         }
         const uint32_t bd = sum(bo);
         const auto key = L::make(exact_d2<SC, D>(p, q), node);
-        bool cand = here && bd <= cull && L::less(key, kth);
+        const bool seen = here && bd < cull;
+        bool cand = seen && L::less(key, kth);
         unsigned m = __ballot_sync(kFull, cand);
+        const E nearest = L::d2(L::shfl(list.key[0], 0));
         while (m) {
           const int src = __ffs(m) - 1;
           insert(L::shfl(key, src));
           cand = cand && lane != src && L::less(key, kth);
           m = __ballot_sync(kFull, cand);
         }
+        if (single && !fa.fcp) {
+          const E now = L::d2(L::shfl(list.key[0], 0));
+          tied = (now < nearest ? 0 : tied) + __popc(__ballot_sync(kFull, seen && L::d2(key) == now));
+          refresh();  // (`tied` went up, or a nearer point began it anew)
+        }
         // the subtrees below: far children, then near ones
         if (lvl + h < levels) {
-          const bool last = here && t == h - 1 && bd <= cull;
+          const bool last = here && t == h - 1 && bd < cull;
           const int lChild = 2 * node + 1;
           float fo[D];
 #pragma unroll
@@ -273,7 +288,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
 #pragma unroll
           for (int side = 0; side < 2; side++) {  // 0: far, 1: near
             const int child = lChild + int(leftIsClose == (side == 0));
-            const bool push = last && child < n && child != skip && (side == 1 || fd <= cull);
+            const bool push = last && child < n && child != skip && (side == 1 || fd < cull);
             const unsigned pm = __ballot_sync(kFull, push);
             if (push) {
               const int at = cnt + __popc(pm & ((1u << lane) - 1u));
@@ -290,7 +305,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
         int pick = -1;
         if (cnt > kBestFirst) {
           while (cnt > 0 && pick < 0) {
-            if (st.dist[cnt - 1] <= cull)
+            if (st.dist[cnt - 1] < cull)
               pick = cnt - 1;
             else
               cnt--;
@@ -306,7 +321,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
             }
           }
           const uint32_t least = __reduce_min_sync(kFull, best);
-          if (least <= cull) pick = __reduce_max_sync(kFull, best == least ? at : -1);
+          if (least < cull) pick = __reduce_max_sync(kFull, best == least ? at : -1);
         }
         if (pick < 0) break;
         curr = st.node[pick];
@@ -329,14 +344,19 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     bool ok = usable;
     const bool filled = L::id(kth) != -1;
     const E X = filled ? L::d2(kth) : r2;
-    if (fa.fcp) {
+    if (single) {
       const auto first = L::shfl(list.key[0], 0);
       const auto second = L::shfl(list.key[0], 1);
-      const bool none = !(L::d2(first) < r2);
-      ok = ok && (none || L::id(second) == -1 || L::d2(first) < L::d2(second));
+      const bool none = fa.fcp ? !(L::d2(first) < r2) : L::id(first) == -1;
+      if (ok && !none && !(L::d2(first) < r2 &&
+                           (L::id(second) == -1 || L::d2(first) < L::d2(second))))
+        ok = !fa.fcp && tied <= kTied &&
+             surely_visited<SC, D, EXPL, VEC>(fa, nd, q, tv.bounds, L::id(first), L::d2(first));
       if (ok && lane == 0) {
+        const E d = none ? r2 : L::d2(first);
         if (a.out_ids) a.out_ids[myq] = none ? -1 : L::id(first);
-        if (a.out_d2) ((E *)a.out_d2)[myq] = none ? r2 : L::d2(first);
+        if (a.out_d2) ((E *)a.out_d2)[myq] = d;
+        if (a.out_max) ((E *)a.out_max)[myq] = d;
       }
     } else {
       bool sure = true;
@@ -383,7 +403,7 @@ template <int SC, int D>
 int launch_warp_layout(const WarpArgs &wa, cudaStream_t st)
 {
   const bool vec = vector_points(wa.f.q, D);
-  const bool one = (wa.f.fcp ? 2 : wa.f.kk) <= 32;
+  const bool one = wa.f.kk <= 32;
 #define CKB_WARP(EXPL_, VEC_)                                                 \
   return one ? launch_warp<SC, D, EXPL_, VEC_, 1>(wa, st)                     \
              : launch_warp<SC, D, EXPL_, VEC_, 4>(wa, st)
