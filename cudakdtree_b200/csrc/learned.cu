@@ -721,8 +721,10 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   a.out_d2 = d_out_d2;
   a.visits = d_visits;
   a.block_size = p->block_size;
-  if ((p->flags & CUKD_QUERY_MORTON) && !order_pays(nq, p->k, L.D, n * L.stride)) {
-    // (in the caller's order)
+  const bool isFloat = L.scalar == CUKD_FLOAT32;
+  const bool packet = (p->flags & CUKD_QUERY_WARP_PACKET) && isFloat && p->k <= 32;
+  if ((p->flags & CUKD_QUERY_MORTON) && !packet && !order_pays(nq, p->k, L.D, n * L.stride)) {
+    // (in the caller's order; the packet kernel's warps need neighbours)
   } else if ((p->flags & CUKD_QUERY_MORTON) && d_world_bounds) {
     CKB_TRY(query_order(d_queries, nq, L.scalar, L.D, d_world_bounds, nullptr, nullptr, &a.order,
                         st, &arena));
@@ -746,8 +748,6 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   fa.fb_list = fb1;
   fa.radius_scale = radius_scale;
   fa.status = d_status;
-  const bool isFloat = L.scalar == CUKD_FLOAT32;
-  const bool packet = (p->flags & CUKD_QUERY_WARP_PACKET) && isFloat && p->k <= 32;
   if (isFloat && p->k <= 32 && !packet) {
     // pass 1: radii predicted and searched in one kernel
     const int D = L.D;

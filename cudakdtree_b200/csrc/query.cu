@@ -258,9 +258,13 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
   const bool plain = !(p->method == CUKD_STACK_FREE && p->eps != 0.f);
   const bool usable = L.scalar == CUKD_FLOAT32 ? a.cutoff == a.cutoff : a.cutoff_d2 >= 0;
   const bool fastOk = exactOk && (!single || (plain && usable));
+  const bool packet = fastOk && (p->flags & CUKD_QUERY_WARP_PACKET) &&
+                      L.scalar == CUKD_FLOAT32 && !single && a.k <= 32;
   // few queries: a warp each (in any order, so without sorting them), and
-  // what it queues by the named traversal
-  if (fastOk && plain && nq <= warp_queries(L.scalar, a.k)) {
+  // what it queues by the named traversal; unless the caller asks for another
+  // kernel or order
+  if (fastOk && plain && !packet && !(p->flags & CUKD_QUERY_TREE_ORDER) &&
+      nq <= warp_queries(L.scalar, a.k)) {
     fast::WarpArgs wa = {};
     fast::FastArgs &fa = wa.f;
     fa.q = a;
@@ -300,8 +304,9 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     CKB_TRY(run_tree_path(a, L.scalar, L.D, levels, codes, vals, st));
     CKB_TRY(radix_sort_pairs(codes, vals, codes2, vals2, nq, levels, st, &arena));
     a.order = (const int32_t *)vals;
-  } else if ((p->flags & CUKD_QUERY_MORTON) && fastOk && !order_pays(nq, a.k, L.D, n * L.stride)) {
-    // (in the caller's order)
+  } else if ((p->flags & CUKD_QUERY_MORTON) && fastOk && !packet &&
+             !order_pays(nq, a.k, L.D, n * L.stride)) {
+    // (in the caller's order; the packet kernel's warps need neighbours)
   } else if ((p->flags & CUKD_QUERY_MORTON) && nq > 1 && narrow && d_world_bounds) {
     CKB_TRY(query_order(d_queries, nq, L.scalar, L.D, d_world_bounds, nullptr, nullptr, &a.order,
                         st, &arena));
@@ -346,8 +351,6 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     CKB_TRY(arena.alloc(&lists, 2 * nq));
     fa.fb_count = ctr;
     fa.fb_list = lists;
-    const bool packet = (p->flags & CUKD_QUERY_WARP_PACKET) && L.scalar == CUKD_FLOAT32 &&
-                        p->k <= 32;
     CKB_TRY(packet ? run_packet(fa, L.D, st) : run_fast(fa, L.scalar, L.D, st));
     wa.f = fa;
     wa.f.q.order = fa.fb_list;
