@@ -232,6 +232,7 @@ struct cukd_batch_plan_s {
   uint32_t *mkeys = nullptr, *mvals = nullptr, *mkeys2 = nullptr, *mvals2 = nullptr;
   uint32_t *mcounts = nullptr;
   int32_t *fb_list = nullptr;
+  int32_t *fb_left = nullptr;  // stack-free lists with eps: queued after the warp kernel
   int64_t maxCloudQueries = 0;  // <= kSegSortMax: per-cloud Morton sort in shared memory
   int *ctr = nullptr;       // [0..1] fast-path counters, [2..4] subtree work counters
   void *lists = nullptr;    // current forest work lists (one block)
@@ -423,12 +424,25 @@ static int query_impl(cukd_batch_plan_s *p, const float *pts, const float *bound
     fa.fb_count = p->ctr + 1;
     fa.fb_list = p->fb_list;
     CKB_TRY(run_fast(fa, CUKD_FLOAT32, D, st));
-    if (p->params.d_reordered_count)
-      CKB_CUDA(cudaMemcpyAsync(p->params.d_reordered_count, fa.fb_count, sizeof(int),
-                               cudaMemcpyDeviceToDevice, st));
     QArgs b = a;
     b.order = p->fb_list;
     b.count_ptr = fa.fb_count;
+    if (p->fb_left) {
+      // lists with eps are the exact ones but at ties, which the warp kernel
+      // tells from distances too close for the fast kernel's keys
+      fast::WarpArgs wa = {};
+      wa.f = fa;
+      wa.f.q = b;
+      wa.f.fb_count = p->ctr;
+      wa.f.fb_list = p->fb_left;
+      wa.queue_limit = INT32_MAX;
+      CKB_TRY(run_warp(wa, CUKD_FLOAT32, D, st));
+      b.order = p->fb_left;
+      b.count_ptr = p->ctr;
+    }
+    if (p->params.d_reordered_count)
+      CKB_CUDA(cudaMemcpyAsync(p->params.d_reordered_count, b.count_ptr, sizeof(int),
+                               cudaMemcpyDeviceToDevice, st));
     b.block_size = std::min(b.block_size, 256);  // reference-order kernels: <= 256 threads
     return run_query(b, CUKD_FLOAT32, D, p->params.method, p->kind, st);
   }
@@ -527,6 +541,8 @@ int cukd_batch_plan_create(cukd_batch_plan **out, int num_dims, int64_t num_clou
   T(dalloc(p, &p->mvals2, std::max<int64_t>(nq, 1)));
   T(dalloc(p, &p->mcounts, radix_sort_counts(std::max<int64_t>(nq, 1))));
   T(dalloc(p, &p->fb_list, std::max<int64_t>(nq, 1)));
+  if (params->method == CUKD_STACK_FREE && params->eps != 0.f)
+    T(dalloc(p, &p->fb_left, std::max<int64_t>(nq, 1)));
   T(dalloc(p, &p->ctr, 8));
   if (rc != CUKD_OK) return fail(rc);
   if (cudaMemcpy(p->d_poff, p->poff.data(), 8 * (B + 1), cudaMemcpyHostToDevice) != cudaSuccess ||

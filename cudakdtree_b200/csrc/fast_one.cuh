@@ -32,6 +32,7 @@ template <> struct Num<0> {
   // bits of a float at or below / at or above a distance of the answer
   __device__ static uint32_t below(E e) { return __float_as_uint(e); }
   __device__ static uint32_t above(E e) { return __float_as_uint(e); }
+  __device__ static E farthest() { return __uint_as_float(0x7f800000u); }
   __device__ static E cutoff(const query::QArgs &a) { return __fmul_rn(a.cutoff, a.cutoff); }
   __device__ static E seeded(E r2, float radius, float scale)
   {
@@ -59,6 +60,7 @@ template <> struct Num<1> {
   __device__ static E exact_add(E a, E b) { return a + b; }
   __device__ static uint32_t below(E e) { return __float_as_uint(__ll2float_rd(e)); }
   __device__ static uint32_t above(E e) { return __float_as_uint(__ll2float_ru(e)); }
+  __device__ static E farthest() { return 0x7fffffffffffffffll; }
   __device__ static E cutoff(const query::QArgs &a) { return a.cutoff_d2; }
   __device__ static E seeded(E r2, float radius, float scale)
   {

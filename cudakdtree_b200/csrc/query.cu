@@ -252,8 +252,7 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
   // FCP and k = 1 have a search that knows ties, too (fcp_fast_one); one that
   // is stack-free with eps may return a point that is not the closest, and
   // one with a NaN or negative cut-off what its traversal makes of that: both
-  // are left to their traversal.  Lists ignore eps but for ties, which the
-  // warp kernel cannot tell from their last point alone.
+  // are left to their traversal.  Lists ignore eps but for ties.
   const bool single = a.k == 1;
   const bool plain = !(p->method == CUKD_STACK_FREE && p->eps != 0.f);
   const bool usable = L.scalar == CUKD_FLOAT32 ? a.cutoff == a.cutoff : a.cutoff_d2 >= 0;
@@ -357,7 +356,9 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     wa.f.q.count_ptr = fa.fb_count;
     wa.f.fb_count = ctr + 1;
     wa.f.fb_list = lists + nq;
-    wa.queue_limit = kWarpQueue;
+    // (a list with eps is the exact one, which its traversal does not give:
+    // however many are queued)
+    wa.queue_limit = plain ? kWarpQueue : INT32_MAX;
     wa.hand_over = true;
     CKB_TRY(run_warp(wa, L.scalar, L.D, st));
     if (p->d_reordered_count)

@@ -124,6 +124,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
   constexpr int kTied = 32;
   const bool single = k == 1;
   const int K = single ? 2 : k;
+  // a stack-free list with eps is its traversal's at ties, else the exact one:
+  // the smallest distance left out tells (`beyond`)
+  const bool eps = !single && fa.method == CUKD_STACK_FREE && a.eps != 0.f;
   // this lane's place in a treelet (lane 31 has none)
   const int t = 31 - __clz(lane + 1);
   for (int64_t w = blockIdx.x * int64_t(kWarpsPerBlock) + wid; w < limit;
@@ -151,7 +154,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
       const bool exclusive = single && L::id(kth) != -1 && (fa.fcp || tied > kTied);
       cull = N::above(L::d2(kth)) + (exclusive ? 0u : 1u);
     };
+    E beyond = N::farthest();  // this lane's share
     auto insert = [&](auto x) {
+      if (eps && L::id(kth) != -1 && L::d2(kth) < beyond) beyond = L::d2(kth);  // pushed out
 #pragma unroll
       for (int i = 0; i < KL; i++) {
         const int pos = __popc(__ballot_sync(kFull, L::less(list.key[i], x)));
@@ -266,12 +271,15 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
         bool cand = seen && L::less(key, kth);
         unsigned m = __ballot_sync(kFull, cand);
         const E nearest = L::d2(L::shfl(list.key[0], 0));
+        bool listed = false;
         while (m) {
           const int src = __ffs(m) - 1;
           insert(L::shfl(key, src));
+          listed = listed || lane == src;
           cand = cand && lane != src && L::less(key, kth);
           m = __ballot_sync(kFull, cand);
         }
+        if (eps && seen && !listed && L::d2(key) < beyond) beyond = L::d2(key);
         if (single && !fa.fcp) {
           const E now = L::d2(L::shfl(list.key[0], 0));
           tied = (now < nearest ? 0 : tied) + __popc(__ballot_sync(kFull, seen && L::d2(key) == now));
@@ -359,13 +367,13 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
         if (a.out_max) ((E *)a.out_max)[myq] = d;
       }
     } else {
-      bool sure = true;
+      bool sure = !(eps && filled) || (X < r2 && X < beyond);
 #pragma unroll
       for (int i = 0; i < KL; i++) {
         const int j = 32 * i + lane;
-        if (ok && j < k && L::id(list.key[i]) != -1 && !(L::d2(list.key[i]) < X))
-          sure = sure && !(fa.method == CUKD_STACK_FREE && a.eps != 0.f) &&
-                 !(fa.method == CUKD_CCT && !tv.bounds) &&
+        if (ok && !(eps && filled) && j < k && L::id(list.key[i]) != -1 &&
+            !(L::d2(list.key[i]) < X))
+          sure = sure && !eps && !(fa.method == CUKD_CCT && !tv.bounds) &&
                  surely_visited<SC, D, EXPL, VEC>(fa, nd, q, tv.bounds, L::id(list.key[i]), X);
       }
       ok = ok && __all_sync(kFull, sure);
