@@ -148,7 +148,8 @@ struct Nodes {
     }
     const int dd = EXPL ? dim_of(node) : lvl % D;
     *dim = dd;
-    return __ldg((const T *)(tree + int64_t(node) * stride + poff) + dd);
+    // (a record whose dim is none of the point's reads as if it were the first)
+    return __ldg((const T *)(tree + int64_t(node) * stride + poff) + (uint32_t(dd) < D ? dd : 0));
   }
 };
 
