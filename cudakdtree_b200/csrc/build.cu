@@ -1408,8 +1408,8 @@ int build_impl(void *pts, int64_t n, const Layout &L, void *worldBounds, cudaStr
   // two key copies, candidates, permutation, dims, records; the rest is what
   // a level's subtrees need
   const size_t w = TempArena::rounded(sizeof(uint32_t) * n);
-  CKB_TRY(arena.reserve((3 * (D + 1) + 1) * w + TempArena::rounded(n) +
-                        TempArena::rounded(size_t(n) * L.stride) + TempArena::rounded(n) + 16384));
+  arena.reserve((3 * (D + 1) + 1) * w + TempArena::rounded(n) +
+                TempArena::rounded(size_t(n) * L.stride) + TempArena::rounded(n) + 16384);
   return build_run<SC, D>(pts, n, L, worldBounds, st, arena);
 }
 

@@ -73,14 +73,14 @@ struct TempArena {
   static size_t rounded(size_t bytes) { return (std::max<size_t>(bytes, 16) + 255) & ~size_t(255); }
   // One block for the allocations that follow (what does not fit it is
   // allocated by itself): twenty stream-ordered allocations of a build cost
-  // the host as much as its launches.
-  int reserve(size_t bytes)
+  // the host as much as its launches.  Without one (a resource may limit the
+  // size of its blocks) each of them is allocated by itself.
+  void reserve(size_t bytes)
   {
     uint8_t *p = nullptr;
-    CKB_TRY(alloc(&p, bytes));
+    if (alloc(&p, bytes) != CUKD_OK) return;
     block = p;
     left = bytes;
-    return CUKD_OK;
   }
   template <typename T>
   int alloc(T **out, size_t count)

@@ -737,9 +737,10 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   int *ctr = nullptr;
   CKB_TRY(arena.alloc(&ctr, 4));
   CKB_CUDA(cudaMemsetAsync(ctr, 0, 4 * sizeof(int), st));
-  int32_t *fb1 = nullptr, *fb2 = nullptr;
+  int32_t *fb1 = nullptr, *fb2 = nullptr, *fb3 = nullptr;
   CKB_TRY(arena.alloc(&fb1, nq));
-  CKB_TRY(arena.alloc(&fb2, 2 * nq));
+  CKB_TRY(arena.alloc(&fb2, nq));
+  CKB_TRY(arena.alloc(&fb3, nq));
   fast::FastArgs fa = {};
   fa.q = a;
   fa.kk = p->k;
@@ -774,7 +775,7 @@ int cukd_knn_learned(const void *d_tree, int64_t n, const cukd_layout *layout,
   fb.q.order = fb1;
   fb.q.count_ptr = ctr + 1;
   fb.fb_count = ctr + 3;
-  fb.fb_list = fb2 + nq;
+  fb.fb_list = fb3;
   fast::WarpArgs wa = {};
   if (!d_visits) {
     wa.f = fb;

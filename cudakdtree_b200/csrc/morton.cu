@@ -161,8 +161,8 @@ int query_order(const void *queries, int64_t n, int scalar, int D, const void *d
 {
   uint32_t *codes = nullptr, *codes2 = nullptr, *vals = nullptr, *vals2 = nullptr,
            *counts = nullptr;
-  CKB_TRY(arena->reserve(4 * TempArena::rounded(sizeof(uint32_t) * n) +
-                         TempArena::rounded(sizeof(uint32_t) * radix_sort_counts(n))));
+  arena->reserve(4 * TempArena::rounded(sizeof(uint32_t) * n) +
+                 TempArena::rounded(sizeof(uint32_t) * radix_sort_counts(n)));
   CKB_TRY(arena->alloc(&codes, n));
   CKB_TRY(arena->alloc(&codes2, n));
   CKB_TRY(arena->alloc(&vals, n));

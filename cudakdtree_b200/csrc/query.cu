@@ -344,18 +344,19 @@ static int common_query(const void *d_tree, int64_t n, const cukd_layout *layout
     fa.fcp = false;
     fa.method = p->method;
     int *ctr = nullptr;
-    int32_t *lists = nullptr;
+    int32_t *queued = nullptr, *left = nullptr;  // (each no larger than the order)
     CKB_TRY(arena.alloc(&ctr, 2));
     CKB_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(int), st));
-    CKB_TRY(arena.alloc(&lists, 2 * nq));
+    CKB_TRY(arena.alloc(&queued, nq));
+    CKB_TRY(arena.alloc(&left, nq));
     fa.fb_count = ctr;
-    fa.fb_list = lists;
+    fa.fb_list = queued;
     CKB_TRY(packet ? run_packet(fa, L.D, st) : run_fast(fa, L.scalar, L.D, st));
     wa.f = fa;
     wa.f.q.order = fa.fb_list;
     wa.f.q.count_ptr = fa.fb_count;
     wa.f.fb_count = ctr + 1;
-    wa.f.fb_list = lists + nq;
+    wa.f.fb_list = left;
     // (a list with eps is the exact one, which its traversal does not give:
     // however many are queued)
     wa.queue_limit = plain ? kWarpQueue : INT32_MAX;
