@@ -1403,7 +1403,13 @@ template <int SC, int D>
 int build_impl(void *pts, int64_t n, const Layout &L, void *worldBounds, cudaStream_t st,
                const cukd_mem_resource *mem)
 {
-  if (n <= kTile) return build_small<SC, D>(pts, n, L, worldBounds, st);
+  // (the small kernel's one CTA permutes the records a word at a time, with
+  // as many in flight as its threads: us, it / the general sequence, float3 in
+  // records of 192, 256 and 1024 bytes: 512 records 64 / 97, 81 / 110,
+  // 204 / 224; 768: 80 / 97, 106 / 115, 286 / 224; 1024: 91 / 102, 125 / 117,
+  // 362 / 231; 300 of 4096 bytes 446 / 667)
+  const bool wide = n > kSmallThreads && n * L.stride > 240 * 1024;
+  if (n <= kTile && !wide) return build_small<SC, D>(pts, n, L, worldBounds, st);
   TempArena arena(st, mem);
   // two key copies, candidates, permutation, dims, records; the rest is what
   // a level's subtrees need
