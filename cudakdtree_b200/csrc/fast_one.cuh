@@ -14,7 +14,9 @@ namespace fast {
 // traversal works with; `exact` the squared distance the answer is made of.
 // Floats: L is the exact distance (the reference's rounding, no FMA
 // contraction).  Ints: every step rounds down, so L never exceeds the exact
-// int64 distance and falls short of it by less than 2^-21 of it; L grows
+// int64 distance and falls short of it by less than (D + 2) 2^-23 of it (a
+// rounding each for the difference, which the square doubles, the square and
+// the additions); L grows
 // with every |coordinate difference|, so a box's L (of its closest point)
 // never exceeds the L of a point inside.
 template <int SC> struct Num;

@@ -144,11 +144,13 @@ __device__ inline void warp_grow(int32_t *lo, int32_t *hi, uint32_t node, bool v
 }
 
 // Grows the boxes of the nodes that this CTA's valid lanes carry prims to.
-// When those nodes span fewer than kGrowSlots consecutive ids (always near
-// the root, where every warp would otherwise hit the same few boxes), the
-// warps' partial boxes are merged in shared memory first and the CTA issues
-// one global atomic per (node, dim, bound); otherwise each warp issues its
-// own (warp_grow).
+// When those nodes' numbers span fewer than kGrowSlots (always near the root,
+// where every warp would otherwise hit the same few boxes), the warps' partial
+// boxes are merged in shared memory first and the CTA issues one global atomic
+// per (node, dim, bound); otherwise each warp issues its own (warp_grow).
+// Deeper levels are mostly the latter: a level's nodes are numbered in the
+// order in which their parents' threads come to a counter, so those of one CTA
+// may lie far apart.
 constexpr int kGrowSlots = 64;
 template <int D>
 __device__ inline void block_grow(int32_t *lo, int32_t *hi, uint32_t node, bool valid,
