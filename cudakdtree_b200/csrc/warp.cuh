@@ -91,7 +91,9 @@ template <int D> struct Pending {
   float off[D][kPending];   // squared offsets of the box's closest point
 };
 
-template <int SC, int D, bool EXPL, bool VEC, int KL>
+// LIST: k >= 2 without eps (compiled apart: the others' bookkeeping costs it
+// 4% of a 27 us call)
+template <int SC, int D, bool EXPL, bool VEC, int KL, bool LIST>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
     knn_warp_kernel(const __grid_constant__ WarpArgs wa)
 {
@@ -122,11 +124,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
   // the smallest id of the tied points (while they are at most kTied: a group
   // of equal points may be the whole tree)
   constexpr int kTied = 32;
-  const bool single = k == 1;
+  const bool single = !LIST && k == 1;
   const int K = single ? 2 : k;
   // a stack-free list with eps is its traversal's at ties, else the exact one:
   // the smallest distance left out tells (`beyond`)
-  const bool eps = !single && fa.method == CUKD_STACK_FREE && a.eps != 0.f;
+  const bool eps = !LIST && !single && fa.method == CUKD_STACK_FREE && a.eps != 0.f;
   // this lane's place in a treelet (lane 31 has none)
   const int t = 31 - __clz(lane + 1);
   for (int64_t w = blockIdx.x * int64_t(kWarpsPerBlock) + wid; w < limit;
@@ -270,7 +272,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
         const bool seen = here && bd < cull;
         bool cand = seen && L::less(key, kth);
         unsigned m = __ballot_sync(kFull, cand);
-        const E nearest = L::d2(L::shfl(list.key[0], 0));
+        const E nearest = LIST ? E(0) : L::d2(L::shfl(list.key[0], 0));
         bool listed = false;
         while (m) {
           const int src = __ffs(m) - 1;
@@ -393,14 +395,14 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
   }
 }
 
-template <int SC, int D, bool EXPL, bool VEC, int KL>
+template <int SC, int D, bool EXPL, bool VEC, int KL, bool LIST>
 int launch_warp(const WarpArgs &wa, cudaStream_t st)
 {
   // at least a block per SM's share of a queue whose length the host does
   // not know; 7 blocks' stacks fit an SM
   int64_t grid = div_up(wa.f.q.nq, kWarpsPerBlock);
   if (wa.f.q.count_ptr) grid = std::min<int64_t>(grid, int64_t(kNumSMs) * 7);
-  knn_warp_kernel<SC, D, EXPL, VEC, KL>
+  knn_warp_kernel<SC, D, EXPL, VEC, KL, LIST>
       <<<unsigned(std::max<int64_t>(1, grid)), 32 * kWarpsPerBlock,
          sizeof(Pending<D>) * kWarpsPerBlock, st>>>(wa);
   CKB_CHECK_LAUNCH();
@@ -412,9 +414,12 @@ int launch_warp_layout(const WarpArgs &wa, cudaStream_t st)
 {
   const bool vec = vector_points(wa.f.q, D);
   const bool one = wa.f.kk <= 32;
-#define CKB_WARP(EXPL_, VEC_)                                                 \
-  return one ? launch_warp<SC, D, EXPL_, VEC_, 1>(wa, st)                     \
-             : launch_warp<SC, D, EXPL_, VEC_, 4>(wa, st)
+  const bool list = wa.f.kk > 1 && !(wa.f.method == CUKD_STACK_FREE && wa.f.q.eps != 0.f);
+#define CKB_WARP(EXPL_, VEC_)                                                       \
+  return list ? (one ? launch_warp<SC, D, EXPL_, VEC_, 1, true>(wa, st)             \
+                     : launch_warp<SC, D, EXPL_, VEC_, 4, true>(wa, st))            \
+              : (one ? launch_warp<SC, D, EXPL_, VEC_, 1, false>(wa, st)            \
+                     : launch_warp<SC, D, EXPL_, VEC_, 4, false>(wa, st))
   if (wa.f.q.doff >= 0) {
     if (vec) CKB_WARP(true, true);
     CKB_WARP(true, false);
