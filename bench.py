@@ -1189,6 +1189,16 @@ def kernel_case(name):
                 t.free()
             t = ck.spatial_build(pts)
             t.knn(q, 16, "cct")
+    elif name in ("fcp", "few"):  # fcp_fast_kernel: 1M on 1M points; knn_warp_kernel: 777, k = 8
+        pts = torch.from_numpy(wl.uniform_points(1_000_000, 3, seed=1)).cuda()
+        wb = ck.build_tree(pts)
+        q = torch.from_numpy(wl.uniform_points(1_000_000 if name == "fcp" else 777, 3,
+                                               seed=2)).cuda()
+        for _ in range(2):
+            if name == "fcp":
+                ck.fcp(pts, q, "stack_free", world_bounds=wb, with_d2=True)
+            else:
+                ck.knn(pts, q, 8, world_bounds=wb)
     elif name == "scatter":  # Morton order of 10M queries
         q = torch.from_numpy(wl.gmm_points(10_000_000, seed=3, sample_seed=4)).cuda()
         for _ in range(2):
@@ -1207,7 +1217,7 @@ def kernel_case(name):
 
 
 KERNEL_CASES = ("knn", "learned", "train", "infer", "heap", "fastint", "accumulate", "spatial",
-                "scatter", "build", "inplace", "bitonic")
+                "fcp", "few", "scatter", "build", "inplace", "bitonic")
 
 
 def config_builders(ck, dev, peak=None):

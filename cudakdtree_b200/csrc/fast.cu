@@ -11,7 +11,9 @@
 // already in the list.  So whenever exactly k points have d2 <= X (the
 // (k+1)-th smallest d2 is strictly greater than X) the reference returns
 // exactly those k points, whatever its visiting order.  The same holds for
-// FCP (FCPResult, fcp.h:179-207) when the smallest d2 is unique.  At a tie
+// FCP (FCPResult, fcp.h:179-207) when the smallest d2 is unique, and of
+// several points at it the first in the traversal's preorder is the answer
+// (fcp_fast_one, fast_one.cuh, which answers k = 1 as well).  At a tie
 // (the (k+1)-th d2 equals X) the reference keeps the tied points of the
 // smallest ids among those it visits; a tied point is visited for certain
 // when no far-side step on its path has a plane/corner distance as large as

@@ -228,7 +228,10 @@ typedef struct cukd_query_params {
   float eps;             /* FcpSearchParams::eps, honoured by CUKD_STACK_FREE */
   int64_t cutoff_d2;     /* int trees: squared cut-off radius (INT64_MAX = none) */
   int32_t flags;         /* CUKD_QUERY_* */
-  int32_t block_size;    /* 0 = default (128); else threads per block, 32..256 */
+  /* 0 = default (128); else threads per block, 32..256, at most what the
+   * kernel is compiled for: 128 for FCP, k = 1 and k = 33..64, 64 for k above
+   * that.  Few queries, which run a warp each, take no notice of it. */
+  int32_t block_size;
   /* optional device int: receives how many queries were re-run in the
    * reference's visiting order (distance ties at the k-th boundary) */
   int32_t *d_reordered_count;
